@@ -279,3 +279,61 @@ def tolerance(case):
         # The hidden activation quantised from its bf16 or from its fp32 values: 0.0113, largest 0.074.
         return {"rel": 3e-2, "max": 0.29}
     return {"rel": 7e-3, "max": 2.4e-2}         # one rounding to bf16: 0.0017, largest 0.0059
+
+
+# ---- the same in 64 bits, in plain torch ------------------------------------------------------------------------
+
+def _wide(q, scale=None):
+    """A matrix in 64 bits; `scale` holds one factor for each block of it."""
+    v = q.double() if scale is None else q.float().double()
+    if scale is not None:
+        f = scale.double()
+        f = f.repeat_interleave(v.shape[-1] // f.shape[-1], -1)
+        v = v * f.repeat_interleave(v.shape[-2] // f.shape[-2], -2)
+    return v
+
+
+def _swiglu_mlp(x, w13, w2):
+    gate, up = (x @ w13.t()).chunk(2, dim=-1)
+    return (torch.nn.functional.silu(gate) * up) @ w2.t()
+
+
+def exact(case, seed):
+    """What `run` returns for these inputs, in 64 bits; None for what is no computed number. The quantisation of
+    activations inside a layer is left out: its error is the layer's own."""
+    kind = case["kind"]
+    if kind == "coll" and case["op"] != "allreduce":
+        return None
+    s = prepare(case, seed)
+    if kind == "ep":
+        # One row for each token that selects an expert, in the order of the tokens.
+        used = (s.idx >= 0).any(dim=1)
+        row = (used.long().cumsum(0) - 1).clamp(min=0)
+        gate = torch.where(s.idx >= 0, s.w, torch.zeros_like(s.w)).double().sum(dim=1, keepdim=True)
+        out = torch.where(used[:, None], gate * s.y[row].double(), 0.0)
+        got = {"rows": None, "expert": None, "gate": None, "token": None, "per_expert": None, "out": out}
+        if case["quantize"]:
+            got["scales"] = None
+        return got
+    if kind == "moe":
+        layer, x, out = s.layer, s.x.double(), torch.zeros(s.x.shape, dtype=torch.float64, device=s.x.device)
+        for e in range(case["experts"]):
+            tok, k = (s.idx == e).nonzero(as_tuple=True)
+            if case["fp8_experts"]:
+                w13, w2 = _wide(layer.w13_q[e], layer.w13_s[e]), _wide(layer.w2_q[e], layer.w2_s[e])
+            else:
+                w13, w2 = _wide(layer.w13[e]), _wide(layer.w2[e])
+            out.index_add_(0, tok, _swiglu_mlp(x[tok], w13, w2) * s.w[tok, k].double()[:, None])
+        return out
+    if kind == "tp":
+        layer = s.layer
+        if case["fp8"]:
+            return _swiglu_mlp(s.x.double(), _wide(layer.w1_q, layer.w1_s), _wide(layer.w2_q, layer.w2_s))
+        return _swiglu_mlp(s.x.double(), _wide(layer.w_gate_up), _wide(layer.w_down))
+    if kind == "gemm":
+        if case["fp8"]:
+            return _wide(s.a, s.a_s) @ _wide(s.b, s.b_s).t()
+        return s.a.double() @ s.b.double().t()
+    total = sum(shm.local_view(s.src, pe).to(torch.float64 if s.src.dtype.is_floating_point else torch.int64)
+                for pe in range(case["pes"]))
+    return [total.to(s.src.dtype) if case["dtype"] == "int32" else total for _ in range(case["pes"])]
