@@ -469,7 +469,7 @@ struct Ag8Args {
 };
 
 template <bool SWIGLU>
-__global__ void __launch_bounds__(gemm8::THREADS + 32, 1)
+__global__ void __launch_bounds__(gemm8::THREADS, 1)
 ag_gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, Ag8Args a) {
   extern __shared__ unsigned char smem_raw[];
   __shared__ gemm8::Shared sh;
@@ -603,7 +603,7 @@ int ag_gemm_fp8(rocshmem_team_t team, const void *x_q, const float *x_s, void *g
   auto launch = [&](auto kernel) -> int {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, gemm8::SMEM_BYTES);
     if (e != cudaSuccess) return static_cast<int>(e);
-    return launch_pes(kernel, sms, gemm8::THREADS + 32, gemm8::SMEM_BYTES, s, true, map_a, map_b, a);
+    return launch_pes(kernel, sms, gemm8::THREADS, gemm8::SMEM_BYTES, s, true, map_a, map_b, a);
   };
   return swiglu ? launch(ag_gemm_fp8_kernel<true>) : launch(ag_gemm_fp8_kernel<false>);
 }

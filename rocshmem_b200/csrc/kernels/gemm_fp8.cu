@@ -132,7 +132,7 @@ struct QuantEpilogue8 {
 };
 
 template <bool A_GATHER>
-__global__ void __launch_bounds__(A_GATHER ? gemm8::GATHER_THREADS : gemm8::THREADS, 1)
+__global__ void __launch_bounds__(gemm8::THREADS, 1)
 grouped_gemm_fp8_swiglu_quant_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                                      const float *a_scale, const float *b_scale, unsigned char *out_q, float *out_s,
                                      const int *offsets, int groups, int n, int k, gemm::GatherSrc src) {
@@ -249,7 +249,7 @@ int grouped_gemm_fp8_swiglu_quant(const void *a_q, const float *a_scale, const i
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (row_index != nullptr) {
     if (int rc = prepare8(grouped_gemm_fp8_swiglu_quant_kernel<true>)) return rc;
-    grouped_gemm_fp8_swiglu_quant_kernel<true><<<device_sm_count(), gemm8::GATHER_THREADS, gemm8::SMEM_BYTES, s>>>(
+    grouped_gemm_fp8_swiglu_quant_kernel<true><<<device_sm_count(), gemm8::THREADS, gemm8::SMEM_BYTES, s>>>(
         map_a, map_b, a_scale, b_scale, static_cast<unsigned char *>(out_q), out_s, offsets, groups, n, k, src);
   } else {
     if (int rc = prepare8(grouped_gemm_fp8_swiglu_quant_kernel<false>)) return rc;

@@ -5,11 +5,20 @@
 //   warp 0      TMA producer, one 128-byte K block (128 e4m3) of a 128 x 256 tile per stage, 4 stages;
 //   warp 1      MMA issuer: the four tcgen05.mma (kind::f8f6f4, K = 32 each) of a K block overwrite one
 //               of two 256-column TMEM buffers, then commit to that buffer's mbarrier;
-//   warps 2..9  accumulate: each thread owns one row and 128 columns (one B scale block) in registers;
+//   warps 2..3  gather producers (A_GATHER) or the scheduler's side role (warp 2);
+//   warps 4..11 accumulate: each thread owns one row and 128 columns (one B scale block) in registers;
 //               per K block it reads the raw partial sums with tcgen05.ld and adds them multiplied by
 //               sa[row, kb] * sb[col block, kb]. Two buffers let the tensor core run one K block ahead.
-// At the end of a tile the registers are converted to bf16 and stored. The CUDA-core work per K block
-// (128 FMAs per thread) takes about half as long as the tensor core needs for the block's MMAs.
+// At the end of a tile the registers are converted to bf16 and stored.
+//
+// The accumulate warps bound the kernel as soon as they need longer for a K block than the tensor core does (512
+// cycles at the dense e4m3 rate). What they spend is the round trip tcgen05.ld -> wait::ld, about 115 cycles whatever the
+// piece (without the additions the kernel was only 8 % faster), so a K block is read in two pieces of 64 columns; the
+// two warps of a scheduler fill each other's gaps. The additions take two columns per instruction
+// (fma.rn.f32x2, the same rounding as two fmaf). 128 + 64 registers are more than an even split of the register
+// file gives to 384 threads, so warps 0..3 hand some over (setmaxnreg): 4 warps x 72 + 8 x 216 = 12 x 168.
+// Measured, 4096 x 4096 x 8192 / 8192 x 8192 x 3584 (L2 flushed): eight pieces of 16 columns, one fmaf a column, 160 / 270
+// us (1721 / 1780 TFLOP/s); pieces of 16 in two register sets 140 / 234 us; two pieces of 64 132 / 219 us (2081 / 2195).
 // Waits are bounded as in gemm_core.cuh.
 #pragma once
 
@@ -34,9 +43,12 @@ constexpr int ACC_WARPS = 8;
 constexpr int EPI_ROW_BYTES = 32 * 2 + 16;              // 32 staged bf16 columns per row, padded
 constexpr int EPI_WARP_BYTES = 32 * EPI_ROW_BYTES;
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + ACC_WARPS * EPI_WARP_BYTES + 1024;
-constexpr int THREADS = 64 + ACC_WARPS * 32;
-constexpr int GATHER_WARPS = 2;                     // registers are granted per four warps: 10 or 12 warps cost the same
-constexpr int GATHER_THREADS = THREADS + GATHER_WARPS * 32;
+constexpr int FIRST_ACC_WARP = 4;                       // a whole warpgroup in front: setmaxnreg works on four warps
+constexpr int GATHER_WARPS = 2;                         // warps 2 and 3
+constexpr int THREADS = (FIRST_ACC_WARP + ACC_WARPS) * 32;
+// Registers per thread: what 384 threads are launched with, and what the two parts of the block hold while they work.
+constexpr int REGS_LAUNCH = 168, REGS_FEED = 72, REGS_ACC = 216;
+static_assert(4 * REGS_FEED + ACC_WARPS * REGS_ACC <= (4 + ACC_WARPS) * REGS_LAUNCH, "setmaxnreg.inc would wait for ever");
 constexpr int TMEM_COLS = 512;
 constexpr unsigned long long WAIT_BUDGET_NS = gemm::WAIT_BUDGET_NS;
 
@@ -61,8 +73,9 @@ struct Shared {
 // operand; they are quantised to e4m3 here (the two threads that hold a row's halves exchange their maxima through
 // shared memory) and written to epi.q_row_ptr(t, row) with the block's scale at epi.scale_ptr(t, row).
 // A_GATHER: the A rows (and their scales) are picked by index: tile row r reads row gather->row_index[t.a_row + r]
-// of gather->base / gather->scales. Two extra warps (threads THREADS .. GATHER_THREADS) copy the rows into the
-// stage with the 128-byte swizzle (cp.async) instead of a TMA load; the kernel must then be launched with GATHER_THREADS.
+// of gather->base / gather->scales. Warps 2 and 3 copy the rows into the stage with the 128-byte swizzle (cp.async)
+// instead of a TMA load.
+// The kernel is compiled for and launched with THREADS threads (__launch_bounds__(THREADS, 1): REGS_LAUNCH registers).
 template <bool SWIGLU, bool LATE_A = false, bool EPI_ADD = false, bool QUANT_OUT = false, bool A_GATHER = false,
           class Scheduler, class Epilogue>
 __device__ __forceinline__ void run(const CUtensorMap *map_a, const CUtensorMap *map_b, const float *a_scale,
@@ -95,6 +108,8 @@ __device__ __forceinline__ void run(const CUtensorMap *map_a, const CUtensorMap 
   sm100::tcgen05_fence_after();
   const uint32_t tmem_base = sh.tmem_base;
 
+  if (warp < FIRST_ACC_WARP) {
+  sm100::setmaxnreg_dec<REGS_FEED>();
   if (warp == 0) {
     if (lane == 0) {
       uint32_t stage = 0, phase = 0;
@@ -143,11 +158,11 @@ __device__ __forceinline__ void run(const CUtensorMap *map_a, const CUtensorMap 
         if (sh.abort_flag) break;
       }
     }
-  } else if (A_GATHER && warp >= 2 + ACC_WARPS) {
+  } else if (A_GATHER) {
     // ---- gather producers: asynchronous 16-byte copies straight into the stage, eight lanes per row (128 contiguous
     // bytes), four rows per instruction, sixteen instructions per stage and warp (warp w serves rows [64 w, 64 w + 64)).
     // No registers hold data, so the warps run as far ahead as the ring has free stages.
-    const int gw = warp - 2 - ACC_WARPS;
+    const int gw = warp - 2;
     const uint32_t c = static_cast<uint32_t>(lane & 7);
     uint32_t stage = 0, phase = 0;
     gemm::Tile t;
@@ -175,10 +190,16 @@ __device__ __forceinline__ void run(const CUtensorMap *map_a, const CUtensorMap 
       }
       if (!ok || sh.abort_flag) break;
     }
-  } else if (warp >= 2 + ACC_WARPS) {
-    sched.side_role();  // optional extra warps (kernels launched with more than THREADS threads)
+  } else if (warp == 2) {
+    sched.side_role();
+  }
+  // What follows the roles is compiled for the launch's share. A warpgroup has to be in step for a second setmaxnreg.
+  __syncwarp();
+  sm100::named_barrier(1, 128);
+  sm100::setmaxnreg_inc<REGS_LAUNCH>();
   } else {
-    const int aw = warp - 2;           // 0..7
+    sm100::setmaxnreg_inc<REGS_ACC>();
+    const int aw = warp - FIRST_ACC_WARP;   // 0..7
     const int quarter = warp & 3;      // TMEM lanes [32 * quarter, +32) are accessible to this warp
     const int half = aw / 4;
     // Plain: this thread owns TMEM columns [128 * half, +128), one B scale block.
@@ -189,9 +210,10 @@ __device__ __forceinline__ void run(const CUtensorMap *map_a, const CUtensorMap 
     uint32_t buf = 0, buf_phase = 0;
     gemm::Tile t;
     for (int iter = 0; sched.get(iter, t) && !sh.abort_flag; ++iter) {
-      float acc[128];
+      // Columns 2 i and 2 i + 1 of this thread's 128, as one f32x2 register pair.
+      unsigned long long acc[64];
 #pragma unroll
-      for (int i = 0; i < 128; ++i) acc[i] = 0.f;
+      for (int i = 0; i < 64; ++i) acc[i] = 0ull;
       const bool row_ok = row < t.rows;
       // Gathered A: the row's scales sit with its source row.
       const size_t a_scale_row = A_GATHER ? static_cast<size_t>(gather->row_index[t.a_row + (row_ok ? row : 0)])
@@ -218,34 +240,37 @@ __device__ __forceinline__ void run(const CUtensorMap *map_a, const CUtensorMap 
           if (!sm100::mbar_wait(&sh.tmem_full[buf], buf_phase, &sh.abort_flag, WAIT_BUDGET_NS)) break;
           sm100::tcgen05_fence_after();
           const uint32_t tbuf = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * BN;
-#pragma unroll
-          for (int c = 0; c < 8; ++c) {
-            uint32_t v[16];
-            // SwiGLU: chunks 0..3 come from the gate columns, 4..7 from the up columns.
-            const uint32_t col = SWIGLU ? (c < 4 ? half * 64 + c * 16 : 128 + half * 64 + (c - 4) * 16) : half * 128 + c * 16;
-            const float s = (SWIGLU && c >= 4) ? scale_u[j] : scale[j];
-            sm100::tmem_ld_32x16(tbuf + col, v);
-            sm100::tmem_ld_wait();
-#pragma unroll
-            for (int i = 0; i < 16; ++i) acc[c * 16 + i] = fmaf(s, __uint_as_float(v[i]), acc[c * 16 + i]);
-          }
-          sm100::tcgen05_fence_before();
+          // SwiGLU: the first half of the thread's columns are gate columns, the second half the matching up columns.
+          const uint32_t col0 = SWIGLU ? half * 64 : half * 128;
+          const uint32_t col2 = SWIGLU ? 128 + half * 64 : half * 128 + 64;
+          const unsigned long long s2 = sm100::pack_f32x2(scale[j], scale[j]);
+          const unsigned long long u2 = SWIGLU ? sm100::pack_f32x2(scale_u[j], scale_u[j]) : s2;
+          uint32_t v[64];
+          sm100::tmem_ld_32x64(tbuf + col0, v);
+          sm100::tmem_ld_wait_for(v);
+          sm100::add_scaled(acc, v, s2);
+          sm100::tmem_ld_32x64(tbuf + col2, v);
+          sm100::tmem_ld_wait_for(v);
+          sm100::tcgen05_fence_before();   // everything has arrived: the buffer may be overwritten
           __syncwarp();
           if (lane == 0) sm100::mbar_arrive(&sh.tmem_empty[buf]);
+          sm100::add_scaled(acc + 32, v, u2);
           buf ^= 1u;
           if (buf == 0) buf_phase ^= 1u;
         }
       }
       if (sh.abort_flag) break;
       constexpr int OUT = SWIGLU ? 64 : 128;   // output columns per thread
-      if (SWIGLU) {
+      float out_v[OUT];
 #pragma unroll
-        for (int i = 0; i < 64; ++i) acc[i] = gemm::silu(acc[i]) * acc[64 + i];
+      for (int i = 0; i < OUT; ++i) {
+        out_v[i] = sm100::half_of_f32x2(acc[i / 2], i & 1);
+        if (SWIGLU) out_v[i] = gemm::silu(out_v[i]) * sm100::half_of_f32x2(acc[32 + i / 2], i & 1);
       }
       if constexpr (EPI_ADD) {
         const float rs = row_ok ? epi.row_scale(t, row) : 0.f;
 #pragma unroll
-        for (int i = 0; i < OUT; ++i) acc[i] *= rs;
+        for (int i = 0; i < OUT; ++i) out_v[i] *= rs;
       }
       const int col0 = half * OUT;
       unsigned char *stg = smem + STAGES * STAGE_BYTES + aw * EPI_WARP_BYTES;
@@ -254,7 +279,7 @@ __device__ __forceinline__ void run(const CUtensorMap *map_a, const CUtensorMap 
         // This thread holds 64 of the row's 128 columns; its partner (same row, other half) sits in another warp.
         float amax = 0.f;
 #pragma unroll
-        for (int i = 0; i < 64; ++i) amax = fmaxf(amax, fabsf(acc[i]));
+        for (int i = 0; i < 64; ++i) amax = fmaxf(amax, fabsf(out_v[i]));
         // Value and "this is tile `iter`" travel in one 8-byte shared-memory store; the partner polls for the tag
         // (bounded, and released by the abort flag: no block-wide barrier that a role that gave up could miss).
         // Two slots alternate: a thread can only be at tile i + 2 once its partner has written tile i + 1, i.e.
@@ -278,7 +303,7 @@ __device__ __forceinline__ void run(const CUtensorMap *map_a, const CUtensorMap 
           unsigned *w = reinterpret_cast<unsigned *>(&pk);
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
-            const float *v = acc + q * 16 + i * 4;
+            const float *v = out_v + q * 16 + i * 4;
             const unsigned lo = __nv_cvt_float2_to_fp8x2(make_float2(v[0] * inv, v[1] * inv), __NV_SATFINITE, __NV_E4M3);
             const unsigned hi = __nv_cvt_float2_to_fp8x2(make_float2(v[2] * inv, v[3] * inv), __NV_SATFINITE, __NV_E4M3);
             w[i] = lo | (hi << 16);
@@ -308,7 +333,7 @@ __device__ __forceinline__ void run(const CUtensorMap *map_a, const CUtensorMap 
           int4 pk;
           __nv_bfloat162 *p2 = reinterpret_cast<__nv_bfloat162 *>(&pk);
 #pragma unroll
-          for (int i = 0; i < 4; ++i) p2[i] = __floats2bfloat162_rn(acc[c * 32 + q * 8 + 2 * i], acc[c * 32 + q * 8 + 2 * i + 1]);
+          for (int i = 0; i < 4; ++i) p2[i] = __floats2bfloat162_rn(out_v[c * 32 + q * 8 + 2 * i], out_v[c * 32 + q * 8 + 2 * i + 1]);
           *reinterpret_cast<int4 *>(stg + lane * EPI_ROW_BYTES + q * 16) = pk;
         }
         __syncwarp();
@@ -339,6 +364,9 @@ __device__ __forceinline__ void run(const CUtensorMap *map_a, const CUtensorMap 
       }
       }
     }
+    __syncwarp();
+    sm100::named_barrier(warp / 4 + 1, 128);
+    sm100::setmaxnreg_dec<REGS_LAUNCH>();
   }
   if (sh.abort_flag) {
     unsigned long long t0;
