@@ -75,11 +75,13 @@ void bind_gemm(py::module_ &m) {
           "grouped_gemm_fp8_blockscaled");
   });
   m.def("ag_gemm_bf16", [](uintptr_t team, uintptr_t x, uintptr_t gathered, uintptr_t flags, uintptr_t b, uintptr_t c,
-                           int m_shard, int N, int K, unsigned epoch, int swiglu, uintptr_t stream) {
+                           int m_shard, int N, int K, unsigned epoch, int swiglu, uintptr_t stream, uintptr_t keep) {
     check(ag_gemm_bf16(reinterpret_cast<rocshmem_team_t>(team), P<void>(x), P<void>(gathered),
                        P<unsigned long long>(flags), P<void>(b), P<void>(c), m_shard, N, K, epoch, swiglu,
-                       P<void>(stream)), "ag_gemm_bf16");
-  });
+                       P<void>(stream), P<void>(keep)), "ag_gemm_bf16");
+  }, py::arg("team"), py::arg("x"), py::arg("gathered"), py::arg("flags"), py::arg("b"), py::arg("c"),
+        py::arg("m_shard"), py::arg("N"), py::arg("K"), py::arg("epoch"), py::arg("swiglu"), py::arg("stream"),
+        py::arg("keep") = 0);
   m.def("ag_gemm_fp8", [](uintptr_t team, uintptr_t x_q, uintptr_t x_s, uintptr_t gq, uintptr_t gs, uintptr_t flags,
                           uintptr_t b_q, uintptr_t b_s, uintptr_t c, int m_shard, int N, int K, unsigned epoch,
                           int swiglu, uintptr_t stream) {

@@ -78,12 +78,16 @@ int grouped_gemm_fp8_scatter_add(const void *a_q, const float *a_scale, const vo
 // symmetric scratch [n_ranks * m_shard, K] into which every member pushes its shard; `flags` holds one
 // 32-bit counter per 128-row block (symmetric, zero-initialised once), `epoch` increases by one per call.
 int ag_gemm_bf16(rocshmem_team_t team, const void *x_shard, void *gathered, unsigned long long *flags,
-                 const void *b, void *c, int m_shard, int n, int k, unsigned epoch, int swiglu, void *stream);
+                 const void *b, void *c, int m_shard, int n, int k, unsigned epoch, int swiglu, void *stream,
+                 void *keep = nullptr);
+// A team of one gathers nothing: its rows are read from x_shard, which may then be any 16-byte aligned device memory,
+// and `keep`, if given, receives a copy of them (teams of one only).
 // GEMM -> reduce-scatter: partial[M, N] = A[M, K_local] * B[N, K_local]^T is produced tile by tile and
 // every tile is stored into the staging buffer of the rank that owns its rows
 // (`staging` symmetric [n_ranks][m_shard, N] bf16); the owner then sums the n_ranks contributions into
 // out [m_shard, N]. M = n_ranks * m_shard. `grid_counter` is one zero-initialised u64 in device memory
-// reserved for this operation, `epoch` increases by one per call (1, 2, ...).
+// reserved for this operation, `epoch` increases by one per call (1, 2, ...). A team of one stores its tiles straight
+// into `out`.
 int gemm_rs_bf16(rocshmem_team_t team, const void *a, const void *b, void *staging, void *out, int m_shard,
                  int n, int k, unsigned long long *grid_counter, unsigned epoch, void *stream);
 

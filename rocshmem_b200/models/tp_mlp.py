@@ -59,9 +59,7 @@ class TensorParallelMLP:
                 stream=None) -> torch.Tensor:
         """Returns this rank's ``[m_shard, d_model]`` rows of the MLP output. ``x_shard=None`` uses
         the current content of :meth:`input_buffer`."""
-        if x_shard is not None:
-            self.input_buffer().copy_(x_shard)
-        self.tp.ag_gemm(self.w_gate_up, out=self.h, swiglu=True, stream=stream)
+        self.tp.ag_gemm(self.w_gate_up, out=self.h, swiglu=True, stream=stream, x=x_shard)
         return self.tp.gemm_rs(self.h, self.w_down, out=out, stream=stream)
 
     __call__ = forward

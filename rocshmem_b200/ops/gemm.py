@@ -200,21 +200,33 @@ class TensorParallelLinear:
         return self._ag[k]
 
     def ag_gemm(self, w: torch.Tensor, out: Optional[torch.Tensor] = None, swiglu: bool = False,
-                stream=None) -> torch.Tensor:
+                stream=None, x: Optional[torch.Tensor] = None) -> torch.Tensor:
         """Uses the current content of :meth:`ag_input` on every rank. ``w [N, K]`` local weight shard.
+        ``x [m_shard, K]``: rows that become that content first.
 
         With ``swiglu`` the weight holds gate rows ``[0, N/2)`` and up rows ``[N/2, N)`` and the result
         is ``silu(gate) * up`` of width ``N / 2`` (the activation is applied in the GEMM epilogue)."""
         _check(w, "w")
         N, K = w.shape
         buf = self._ag_buffers(K)
-        x, gathered, flags = buf[0], buf[1], buf[2]
+        rows, gathered, flags = buf[0], buf[1], buf[2]
+        keep = 0
+        if x is not None:
+            # With a team of one the kernel reads the rows where they are and copies them beside its arithmetic. Rows
+            # that the kernel cannot read as they are, or that the call's stream does not own, are copied first.
+            if (self.n_ranks == 1 and x.dtype == torch.bfloat16 and x.shape == rows.shape and x.device == rows.device
+                    and x.is_contiguous() and x.data_ptr() % 16 == 0 and not x.requires_grad
+                    and _stream(stream) == torch.cuda.current_stream().cuda_stream):
+                if x.data_ptr() != rows.data_ptr():
+                    rows, keep = x, rows.data_ptr()
+            else:
+                rows.copy_(x)
         buf[3] += 1
         if out is None:
             out = torch.empty((self.n_ranks * self.m_shard, N // 2 if swiglu else N), dtype=torch.bfloat16,
                               device=w.device)
-        rt._C().ag_gemm_bf16(self.team.handle, x.data_ptr(), gathered.data_ptr(), flags.data_ptr(), w.data_ptr(),
-                             out.data_ptr(), self.m_shard, N, K, buf[3], int(swiglu), _stream(stream))
+        rt._C().ag_gemm_bf16(self.team.handle, rows.data_ptr(), gathered.data_ptr(), flags.data_ptr(), w.data_ptr(),
+                             out.data_ptr(), self.m_shard, N, K, buf[3], int(swiglu), _stream(stream), keep)
         self.kernel_launches += 1
         return out
 

@@ -96,3 +96,35 @@ def test_tp_mlp_fp8_single_rank(shm, d_model, d_ff, m):
         assert gemm.gemm_error_count() == before
         err = (out.float().cpu() - want).abs().max().item()
         assert err <= 5e-2 * want.abs().max().item() + 0.05, (rep, err)
+
+
+@pytest.mark.parametrize("m", [256, 384])
+def test_tp_mlp_alone_reads_the_rows_where_they_are(shm, m):
+    """A team of one: rows in ordinary memory, strided rows and results that share memory with an operand give what the
+    input buffer gives, and the rows are the input buffer's content afterwards."""
+    from rocshmem_b200.models import tp_mlp
+    d = 512
+    mlp = tp_mlp.TensorParallelMLP(d, d, m, seed=4)
+    x = (torch.randn(m, d, generator=torch.Generator().manual_seed(m)) * 0.5).to(torch.bfloat16).cuda()
+    mlp.input_buffer().copy_(x)
+    want = mlp().clone()
+    mlp.input_buffer().zero_()
+    assert torch.equal(mlp(x), want)
+    assert torch.equal(mlp.input_buffer(), x)
+    assert torch.equal(mlp(x.t().contiguous().t()), want)          # strided: copied first
+    assert torch.equal(mlp(x.float()), want)                       # another type: converted first
+    y = x.clone()
+    assert mlp(y, out=y) is y and torch.equal(y, want)
+    # The two kernels with their result over an operand.
+    h = mlp.tp.ag_gemm(mlp.w_gate_up, swiglu=True).clone()
+    mlp.tp.ag_gemm(mlp.w_gate_up, out=mlp.input_buffer(), swiglu=True)
+    assert torch.equal(mlp.input_buffer(), h)
+    assert torch.equal(mlp.tp.gemm_rs(h, mlp.w_down, out=h), want)
+    # A call on another stream than the current one.
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        out = mlp(x)
+    clean(shm)
+    assert torch.equal(out, want)
+    mlp.destroy()
