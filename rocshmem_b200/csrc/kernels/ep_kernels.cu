@@ -11,8 +11,10 @@
 //   C. rows are quantised to e4m3 with one fp32 scale per 128 elements in registers (amax by shuffles
 //      inside 8-lane groups) and stored with 16-byte peer stores straight into their final rows of the
 //      destinations' receive buffers, together with the scales and a 128-byte metadata record. There is
-//      no receiver-side copy. Two ways of sharing the work:
+//      no receiver-side copy. Three ways of sharing the work:
 //        fixed shares   a warp owns whole tokens of its block and sends each to all its destinations;
+//        one rank       a team of one: fixed shares whose rows a warp streams batch by batch (4096 tokens of 7168 in e4m3,
+//                       in a loop: dispatch 35 -> 25 us, combine, whose loads were as many as for four sources, 39 -> 29);
 //        pairs          warps take (token, destination) pairs from per-destination counters, so that no warp is
 //                       left with eight destinations while another has one; a row is quantised again for every
 //                       destination (re-reading it from L2 costs less than a staging pass that idles the links);
@@ -247,7 +249,6 @@ template <bool STAGED>
 __global__ void __launch_bounds__(kEpThreads, 1) ep_dispatch_kernel(DispatchArgs a) {
   // masks [tpb] u64, ranks among the block's tokens per destination [tpb][P] int, pair ranks [tpb][K] int
   extern __shared__ __align__(16) unsigned char s_dyn[];
-  __shared__ int s_rank_cnt[EP_MAX_RANKS];
   __shared__ int s_blk_base[EP_MAX_RANKS];
   __shared__ int s_total[EP_MAX_RANKS];
   __shared__ int s_base[EP_MAX_RANKS];
@@ -298,41 +299,59 @@ __global__ void __launch_bounds__(kEpThreads, 1) ep_dispatch_kernel(DispatchArgs
   unsigned long long *work = STAGED ? rebase(a.buf.work_counter) + EP_WORK_DISPATCH : nullptr;
   if (STAGED && b == 0 && tid < EP_MAX_RANKS) work[(parity ^ 1) * EP_MAX_RANKS + tid] = 0;  // for the next call
 
+  const unsigned warp = tid / 32, lane = tid % 32, nwarps = nthr / 32;
+  // One rank: every token has at most one destination, so a warp streams its rows through 16 vectors a lane, each
+  // reloaded for the next batch as soon as it has been used, and the first batch does not wait for the routing.
+  // Slot s of a row is one vector a lane; two neighbouring ones hold the 16 elements that are quantised together.
+  const bool alone = !STAGED && P == 1;
+  const int row_slots = H / 256;
+  int4 raw[16];
+  auto slot_vec = [&](int s) { return a.cfg.quantize ? (s >> 1) * 64 + int(lane) * 2 + (s & 1) : s * 32 + int(lane); };
+  if (alone && t0 + int(warp) < t1) {
+    const int4 *row = reinterpret_cast<const int4 *>(x + size_t(t0 + warp) * H);
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      if (j < row_slots) raw[j] = row[slot_vec(j)];
+    }
+  }
+
   // ---- A: routing scan ------------------------------------------------------------------------------
-  for (unsigned i = tid; i < EP_MAX_RANKS; i += nthr) s_rank_cnt[i] = 0;
   for (unsigned i = tid; i < unsigned(E); i += nthr) s_exp_cnt[i] = 0;
+  for (int i = tid; i < t1 - t0; i += nthr) s_mask[i] = 0;
   if (tid == 0) s_ok = 1;
   __syncthreads();
-  for (int tok = t0 + tid; tok < t1; tok += nthr) {
-    unsigned long long mask = 0;
-    for (int k = 0; k < K; ++k) {
-      const int e = topk_idx[size_t(tok) * K + k];
-      int rank = 0;
-      if (e >= 0 && e < E) {
-        mask |= 1ull << (e / epr);
-        rank = atomicAdd(&s_exp_cnt[e], 1);
-      }
-      s_pair_rank[(tok - t0) * K + k] = rank;
+  // One thread per (token, k) pair, so that the block's few hundred indices are one memory round trip (a thread per
+  // token made it K dependent ones: 4.2 us of the scan on 4096 tokens of 8 experts).
+  for (int i = tid; i < (t1 - t0) * K; i += nthr) {
+    const int e = topk_idx[size_t(t0) * K + i];
+    int rank = 0;
+    if (e >= 0 && e < E) {
+      atomicOr(&s_mask[i / K], 1ull << (e / epr));
+      rank = atomicAdd(&s_exp_cnt[e], 1);
     }
-    tok_mask[tok] = mask;
-    s_mask[tok - t0] = mask;
-    for (unsigned long long m = mask; m; m &= m - 1) atomicAdd(&s_rank_cnt[__ffsll(static_cast<long long>(m)) - 1], 1);
+    s_pair_rank[i] = rank;
   }
   __syncthreads();
-  for (unsigned d = tid; d < unsigned(P); d += nthr) blk_cnt[b * P + d] = s_rank_cnt[d];
+  for (int i = tid; i < t1 - t0; i += nthr) tok_mask[t0 + i] = s_mask[i];
   for (unsigned e = tid; e < unsigned(E); e += nthr) {
     s_exp_base[e] = s_exp_cnt[e] ? atomicAdd(&exp_cnt[parity * E + e], s_exp_cnt[e]) : 0;
   }
   // Position of every token of the block among the block's tokens that go to the same rank (does not
-  // depend on other blocks, so it is done before the grid barrier).
-  for (unsigned d = tid; d < unsigned(P); d += nthr) {
+  // depend on other blocks, so it is done before the grid barrier). A warp per rank, 32 tokens at a time.
+  for (unsigned d = warp; d < unsigned(P); d += nwarps) {
     int running = 0;
-    for (int i = 0; i < t1 - t0; ++i) {
-      s_rank_in_block[i * P + d] = running;
-      running += static_cast<int>((s_mask[i] >> d) & 1ull);
+    for (int i0 = 0; i0 < t1 - t0; i0 += 32) {
+      const int i = i0 + int(lane);
+      const bool goes = i < t1 - t0 && ((s_mask[i] >> d) & 1ull);
+      const unsigned votes = __ballot_sync(0xffffffffu, goes);
+      if (i < t1 - t0) s_rank_in_block[i * P + d] = running + __popc(votes & ((1u << lane) - 1u));
+      running += __popc(votes);
     }
-    s_blk_base[d] = 0;
-    s_total[d] = 0;
+    if (lane == 0) {
+      blk_cnt[b * P + d] = running;
+      s_blk_base[d] = 0;
+      s_total[d] = 0;
+    }
   }
   if (stamp) phase_ns[1] = detail::now_ns();
   if (!grid_barrier(grid_counter, ++round, B)) return;
@@ -362,7 +381,6 @@ __global__ void __launch_bounds__(kEpThreads, 1) ep_dispatch_kernel(DispatchArgs
       exp_cnt[(parity ^ 1) * E + e] = 0;  // cleared for the next call
     }
   }
-  const unsigned warp = tid / 32, lane = tid % 32, nwarps = nthr / 32;
   const int iters = H / 512;
   const int nscale = H / 128;
   constexpr int kBatch = 8;  // iterations (of 512 elements) whose loads are issued together
@@ -475,6 +493,74 @@ __global__ void __launch_bounds__(kEpThreads, 1) ep_dispatch_kernel(DispatchArgs
         remote_ptr(recv_meta + size_t(slot) * EP_META_WORDS, w)[lane] = word;
         next = __shfl_sync(0xffffffffu, after, 0);
       }
+    }
+  } else if (alone) {
+    // ---- C (one rank): the rows of a warp's tokens as one stream of batches -------------------------------------
+    int tok = t0 + int(warp), s0 = 0, word = 0;   // word: this lane's part of the token's record, or its expert
+    while (tok < t1) {
+      const bool last = s0 + 16 >= row_slots;
+      const int next_tok = last ? tok + int(nwarps) : tok, next_s0 = last ? 0 : s0 + 16;
+      const bool more = next_tok < t1;
+      const int4 *next_row = reinterpret_cast<const int4 *>(x + size_t(more ? next_tok : tok) * H);
+      const int slot = s_mask[tok - t0] ? s_base[0] + s_blk_base[0] + s_rank_in_block[tok - t0] : -1;
+      if (s0 == 0) {
+        word = 0;
+        if (lane < unsigned(EP_MAX_TOPK)) {
+          word = lane < unsigned(K) ? topk_idx[size_t(tok) * K + lane] : -1;
+        } else if (lane < unsigned(EP_META_WEIGHT + K)) {
+          word = __float_as_int(topk_w[size_t(tok) * K + lane - EP_META_WEIGHT]);
+        } else if (lane == unsigned(EP_META_SRC_TOKEN)) {
+          word = tok;
+        } else if (lane == unsigned(EP_META_SRC_RANK)) {
+          word = me;
+        } else if (lane >= unsigned(EP_META_RANK) && lane < unsigned(EP_META_RANK + K)) {
+          word = topk_idx[size_t(tok) * K + lane - EP_META_RANK];
+        }
+      }
+      if (a.cfg.quantize) {
+        int4 *dst = reinterpret_cast<int4 *>(recv_x + size_t(max(slot, 0)) * H);
+#pragma unroll
+        for (int j = 0; j < 16; j += 2) {
+          int4 q;
+          float scale;
+          if (s0 + j < row_slots) q = quantize16(raw[j], raw[j + 1], &scale);
+          if (more && next_s0 + j < row_slots) {
+            raw[j] = next_row[slot_vec(next_s0 + j)];
+            raw[j + 1] = next_row[slot_vec(next_s0 + j + 1)];
+          }
+          if (slot >= 0 && s0 + j < row_slots) {
+            dst[(s0 + j) / 2 * 32 + lane] = q;
+            if ((lane & 7) == 0) s_scales[warp][(s0 + j) * 2 + lane / 8] = scale;
+          }
+        }
+      } else {
+        int4 *dst = reinterpret_cast<int4 *>(recv_x + size_t(max(slot, 0)) * H * 2);
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          if (slot >= 0 && s0 + j < row_slots) dst[slot_vec(s0 + j)] = raw[j];
+          if (more && next_s0 + j < row_slots) raw[j] = next_row[slot_vec(next_s0 + j)];
+        }
+      }
+      if (last) {
+        if (lane == 0) sent_slot[tok] = slot;
+        __syncwarp();
+        if (slot >= 0) {
+          if (a.cfg.quantize && lane < unsigned(nscale / 4)) {
+            reinterpret_cast<float4 *>(recv_scales + size_t(slot) * nscale)[lane] =
+                reinterpret_cast<const float4 *>(s_scales[warp])[lane];
+          }
+          const bool valid = word >= 0 && word < E;
+          if (lane < unsigned(EP_MAX_TOPK)) {
+            word = valid ? word : -1;
+          } else if (lane >= unsigned(EP_META_RANK) && lane < unsigned(EP_META_RANK + K)) {
+            word = valid ? s_exp_base[word] + s_pair_rank[(tok - t0) * K + lane - EP_META_RANK] : 0;
+          }
+          recv_meta[size_t(slot) * EP_META_WORDS + lane] = word;
+        }
+        __syncwarp();
+      }
+      tok = next_tok;
+      s0 = next_s0;
     }
   } else {
   // ---- C (fixed shares): quantise and send, one warp per token ---------------------------------------------
@@ -801,7 +887,9 @@ __device__ __forceinline__ void combine_row(int4 *dst, const int4 **src, const f
 
 // DYNAMIC: warps take tokens from a device-wide counter (a token costs as many remote rows as it has sources, one
 // to eight, so fixed shares differ a lot); the counter only grows, the host tells every call where it starts.
-template <bool DYNAMIC>
+// ALONE: a team of one, so a token has one source row at most, and all 16 loads in flight belong to it (as one of four
+// possible sources it had four: 4096 rows of 14 KiB took 27 us, 4.4 TB/s).
+template <bool DYNAMIC, bool ALONE = false>
 __global__ void __launch_bounds__(kCombineThreads, 1) ep_combine_kernel(CombineArgs a) {
   __shared__ const int4 *s_src[kCombineThreads / 32][EP_MAX_TOPK];
   __shared__ float s_wgt[kCombineThreads / 32][EP_MAX_TOPK];
@@ -878,7 +966,9 @@ __global__ void __launch_bounds__(kCombineThreads, 1) ep_combine_kernel(CombineA
     }
     __syncwarp();
     int4 *dst = reinterpret_cast<int4 *>(out + size_t(tok) * H);
-    if (n_src <= 4) {
+    if (ALONE) {
+      combine_row<1, 16>(dst, src, wgt, n_src, vbegin, vend, lane);
+    } else if (n_src <= 4) {
       combine_row<4, 4>(dst, src, wgt, n_src, vbegin, vend, lane);
     } else {
       combine_row<8, 2>(dst, src, wgt, n_src, vbegin, vend, lane);
@@ -1009,7 +1099,9 @@ int ep_dispatch(rocshmem_team_t team, const EpConfig &cfg, const EpBuffers &buf,
   const int tpb = (cfg.max_tokens + cfg.blocks - 1) / cfg.blocks;
   const size_t smem = size_t(tpb) * ((ht->world.size + cfg.top_k) * sizeof(int) + sizeof(unsigned long long));
   if (smem > 40 * 1024) return cudaErrorInvalidValue;  // use more blocks for this many tokens
-  if (cfg.dynamic) {
+  // Handing out (token, destination) pairs levels shares of unequal size; with one rank they are equal, and the counters
+  // and the second grid barrier cost more than they give (4096 tokens: 43 us against 41, 611: 25 against 20).
+  if (cfg.dynamic && ht->world.size > 1) {
     if (!buf.work_counter || !buf.stage_meta || !buf.item_tok) return cudaErrorInvalidValue;
     return launch_pes(ep_dispatch_kernel<true>, cfg.blocks, kEpThreads, smem, static_cast<cudaStream_t>(stream), true,
                       a);
@@ -1027,6 +1119,7 @@ int ep_combine(rocshmem_team_t team, const EpConfig &cfg, const EpBuffers &buf, 
   if (int rc = validate(cfg, ht->world.size, num_tokens)) return rc;
   CombineArgs a{cfg, buf, static_cast<const __nv_bfloat16 *>(y), static_cast<__nv_bfloat16 *>(out), topk_idx,
                 topk_w, num_tokens, weighted, team, combine_calls_base, 1, 1};
+  const bool alone = ht->world.size == 1;
   if (cfg.low_latency) {
     // Four warps per token, one token per block of 128 threads, no closing barrier.
     a.split = (cfg.hidden / 8) % 4 == 0 ? 4 : 1;
@@ -1035,7 +1128,14 @@ int ep_combine(rocshmem_team_t team, const EpConfig &cfg, const EpBuffers &buf, 
     if (rt.n_local() > 1) {
       blocks = std::min(blocks, coresident_blocks_per_pe(ep_combine_kernel<false>, kLlThreads, 0, rt.n_local()));
     }
-    return launch_pes(ep_combine_kernel<false>, blocks, kLlThreads, 0, static_cast<cudaStream_t>(stream), false, a);
+    return launch_pes(alone ? ep_combine_kernel<false, true> : ep_combine_kernel<false>, blocks, kLlThreads, 0,
+                      static_cast<cudaStream_t>(stream), false, a);
+  }
+  if (alone) {
+    // Tokens cost the same, so they need no counter; two warps share a token, which halves the last round.
+    if (cfg.hidden >= 2048) a.split = 2;
+    return launch_pes(ep_combine_kernel<false, true>, cfg.blocks, kCombineThreads, 0, static_cast<cudaStream_t>(stream),
+                      false, a);
   }
   if (cfg.dynamic) {
     if (buf.work_counter == nullptr) return cudaErrorInvalidValue;

@@ -128,3 +128,48 @@ def test_tp_mlp_alone_reads_the_rows_where_they_are(shm, m):
     clean(shm)
     assert torch.equal(out, want)
     mlp.destroy()
+
+
+@pytest.mark.parametrize("T", [1, 149, 700])
+@pytest.mark.parametrize("H,K,quantize", [(512, 3, True), (4096, 8, True), (4608, 1, True), (7168, 8, True),
+                                          (512, 8, False), (4096, 6, False), (8192, 2, False)])
+def test_dispatch_and_combine_of_a_rank_on_its_own(shm, T, H, K, quantize):
+    """A team of one streams its rows: sizes around the stream's batches (16 vectors a lane: 4096 elements), fewer and
+    more tokens than blocks, tokens without an expert. Rows, scales and records come out exactly; the combined rows are
+    one fp32 product rounded to bf16."""
+    from rocshmem_b200.ops import moe
+    E = 16
+    g = torch.Generator().manual_seed(T * 7 + H)
+    x = torch.randn(T, H, generator=g).to(torch.bfloat16).cuda()
+    idx, w = moe.make_routing(T, E, K, T + H)
+    idx[::5, -1] = -1
+    if T > 3:
+        idx[3] = -1
+    idx, w = idx.cuda(), w.cuda()
+    d = moe.EpDispatcher(E, K, H, max(T, 200), quantize=quantize)
+    used = (idx >= 0).any(dim=1)
+    n = int(used.sum())
+    for rep in range(2):
+        r = d.dispatch(x, idx, w)
+        clean(shm)
+        assert r.num_rows() == n and r.row_ranges() == [(0, n)]
+        assert torch.equal(r.src_token()[:n].long(), used.nonzero().flatten())
+        assert torch.equal(r.local_expert_idx()[:n], idx[used])
+        assert torch.equal(r.gate_weights()[:n], w[used])
+        assert torch.equal(r.rows_per_expert()[:E].long(), torch.bincount(idx[idx >= 0].long(), minlength=E))
+        if quantize:
+            q, s = moe.fp8_quantize_1x128(x[used])
+            assert torch.equal(r.recv_x[:n].view(torch.uint8), q.view(torch.uint8))
+            assert torch.equal(r.recv_scales[:n], s)
+        else:
+            assert torch.equal(r.recv_x[:n], x[used])
+        y = d.result_buffer()
+        y[:n].copy_(torch.randn(n, H, generator=g).to(torch.bfloat16))
+        gate = torch.where(idx >= 0, w, torch.zeros_like(w)).sum(dim=1)
+        for weighted in (True, False):
+            out = d.combine(y, idx, w, T, weighted=weighted)
+            want = torch.zeros(T, H, device="cuda")
+            want[used] = y[:n].float() * (gate[used, None] if weighted else 1.0)
+            clean(shm)
+            assert (out.float() - want).abs().max().item() <= 2 ** -8 * want.abs().max().item()   # one bf16 rounding
+    d.destroy()
