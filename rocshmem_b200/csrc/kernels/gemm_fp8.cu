@@ -7,6 +7,7 @@
 
 #include "gemm_fp8_core.cuh"
 #include "gemm_kernels.hpp"
+#include "gemm_split_core.cuh"
 #include "gemm_tmap.hpp"
 #include "launch.cuh"
 
@@ -55,6 +56,15 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   sched.tiles = ((m + gemm8::BM - 1) / gemm8::BM) * sched.tiles_n;
   RowMajorEpilogue8 epi{c, static_cast<size_t>(n)};
   gemm8::run<false, false>(&map_a, &map_b, a_scale, b_scale, k / gemm8::KB, sched, epi, smem_raw, sh);
+}
+
+// Few tiles: a cluster shares a tile's K (gemm_split_core.cuh).
+template <int BN>
+__global__ void __launch_bounds__(gemms::threads(BN), 1)
+gemm_fp8_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, gemms::Args a) {
+  extern __shared__ unsigned char smem_raw[];
+  __shared__ gemms::Shared sh;
+  gemms::run<true, BN>(&map_a, &map_b, a, smem_raw, sh);
 }
 
 constexpr int kMaxGroups8 = 256;
@@ -201,6 +211,12 @@ int gemm_fp8_blockscaled(const void *a_q, const float *a_scale, const void *b_q,
   // K blocks are consumed four at a time; B scale blocks cover 128 rows of B.
   if (m <= 0 || n <= 0 || k <= 0 || (k % 512) != 0 || (n % 128) != 0) return cudaErrorInvalidValue;
   CUtensorMap map_a, map_b;
+  // As many 128 x 128 tiles as SMs at most: clusters that share a tile's K.
+  const int rc = gemms::try_launch<gemm_fp8_split_kernel<128>, gemm_fp8_split_kernel<64>>(
+      a_q, b_q, c, a_scale, b_scale, m, n, k, 2,
+      [k](CUtensorMap *map, const void *base, int rows, int box) { return encode_tmap_2d(map, base, rows, k, 1, box); },
+      static_cast<cudaStream_t>(stream));
+  if (rc != -2) return rc;
   if (!encode_tmap_2d(&map_a, a_q, m, k, 1, gemm8::BM) || !encode_tmap_2d(&map_b, b_q, n, k, 1, gemm8::BN / 2)) return -1;
   const int tiles = ((m + gemm8::BM - 1) / gemm8::BM) * ((n + gemm8::BN - 1) / gemm8::BN);
   const int grid = std::min(tiles, device_sm_count());

@@ -9,6 +9,7 @@
 #include "gemm_core.cuh"
 #include "gemm2_core.cuh"
 #include "gemm_kernels.hpp"
+#include "gemm_split_core.cuh"
 #include "gemm_tmap.hpp"
 #include "launch.cuh"
 
@@ -111,6 +112,15 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
   sched.tiles = ((m + 2 * gemm2::BM - 1) / (2 * gemm2::BM)) * sched.tiles_n;
   RowMajorEpilogue epi{c, static_cast<size_t>(n)};
   gemm2::run<false>(&map_a, &map_b, k * 2, sched, epi, smem_raw, sh);
+}
+
+// ---- plain GEMM with few tiles: a cluster shares a tile's K --------------------------------------------------------
+template <int BN>
+__global__ void __launch_bounds__(gemms::threads(BN), 1)
+gemm_bf16_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, gemms::Args a) {
+  extern __shared__ unsigned char smem_raw[];
+  __shared__ gemms::Shared sh;
+  gemms::run<false, BN>(&map_a, &map_b, a, smem_raw, sh);
 }
 
 // ---- grouped GEMM ------------------------------------------------------------------------------------------------
@@ -260,13 +270,21 @@ int gemm_bf16_pair(const void *a, const void *b, void *c, int m, int n, int k, v
 
 int gemm_bf16_one_cta(const void *a, const void *b, void *c, int m, int n, int k, void *stream);
 
-// More than one 128-row block: two CTAs per 256 x 256 tile (about 10 % faster, see gemm2_core.cuh), unless
+// As many 128 x 128 tiles as SMs at most: clusters that share a tile's K (gemm_split_core.cuh). More tiles, and more
+// than one 128-row block: two CTAs per 256 x 256 tile (about 10 % faster, see gemm2_core.cuh), unless
 // ROCSHMEM_GEMM_TWO_CTA=0 asks for the one-CTA kernel.
 int gemm_bf16(const void *a, const void *b, void *c, int m, int n, int k, void *stream) {
   static const bool two_cta = [] {
     const char *e = std::getenv("ROCSHMEM_GEMM_TWO_CTA");
     return e == nullptr || e[0] != '0';
   }();
+  if (m > 0 && n > 0 && k > 0 && k % 8 == 0) {
+    const int rc = gemms::try_launch<gemm_bf16_split_kernel<128>, gemm_bf16_split_kernel<64>>(
+        a, b, c, nullptr, nullptr, m, n, k * 2, 1,
+        [k](CUtensorMap *map, const void *base, int rows, int box) { return encode_tmap_2d(map, base, rows, k, 2, box); },
+        static_cast<cudaStream_t>(stream));
+    if (rc != -2) return rc;
+  }
   if (two_cta && m > gemm::BM && device_sm_count() % 2 == 0) return gemm_bf16_pair(a, b, c, m, n, k, stream);
   return gemm_bf16_one_cta(a, b, c, m, n, k, stream);
 }

@@ -339,3 +339,41 @@ def test_headline_shapes_in_full(kind):
             lo += sz
     assert gemm.gemm_error_count() == before
 
+
+
+@pytest.mark.parametrize("m", [1, 8, 9, 63, 127, 128, 129, 300])
+@pytest.mark.parametrize("n,k", [(8, 64), (1001, 520), (2048, 4096), (4104, 2056)])
+def test_gemm_bf16_few_tiles(m, n, k):
+    """Products with few tiles: a cluster shares a tile's K. Row counts around the boxes of A, widths that are no
+    multiple of a tile or of 16 bytes, K that the cluster's CTAs do not divide evenly."""
+    from rocshmem_b200.ops import gemm
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+    a = torch.randn(m, k, generator=g, device="cuda").to(torch.bfloat16)
+    b = (torch.randn(n, k, generator=g, device="cuda") * k ** -0.5).to(torch.bfloat16)
+    before = gemm.gemm_error_count()
+    out = torch.full((m + 1, n), 7.0, dtype=torch.bfloat16, device="cuda")
+    gemm.gemm_bf16(a, b, out=out[:m])
+    torch.cuda.synchronize()
+    assert gemm.gemm_error_count() == before
+    want = a.double() @ b.double().t()
+    # bf16 rounding (2^-9 relative) and fp32 sums of k products, whose magnitudes add up to about sqrt(k) * 0.8
+    assert ((out[:m].double() - want).abs() <= 2 ** -8 * want.abs() + 2 ** -23 * k).all()
+    assert torch.all(out[m] == 7.0), "rows past the result were written"
+    again = gemm.gemm_bf16(a, b)
+    assert torch.equal(again, out[:m]), "the order of the sum is fixed"
+
+
+@pytest.mark.parametrize("m", [1, 9, 64, 127, 128, 200])
+@pytest.mark.parametrize("n,k", [(128, 512), (640, 1536), (2048, 7168), (7168, 2048)])
+def test_gemm_fp8_few_tiles(m, n, k):
+    """The same for block-scaled e4m3 operands."""
+    from rocshmem_b200.ops import gemm
+    a_q, a_s, b_q, b_s, a_deq, b_deq = _fp8_inputs(m, n, k, seed=m + n)
+    before = gemm.gemm_error_count()
+    out = gemm.gemm_fp8_blockscaled(a_q, a_s, b_q, b_s)
+    torch.cuda.synchronize()
+    assert gemm.gemm_error_count() == before
+    want = a_deq.double() @ b_deq.double().t()
+    size = (a_deq.double().abs() @ b_deq.double().abs().t())       # what the rounding of the sums scales with
+    assert ((out.double() - want).abs() <= 2 ** -8 * want.abs() + 2 ** -17 * size).all()
+    assert torch.equal(gemm.gemm_fp8_blockscaled(a_q, a_s, b_q, b_s), out)
