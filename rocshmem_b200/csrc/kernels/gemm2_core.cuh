@@ -192,10 +192,11 @@ __device__ __forceinline__ void run(const CUtensorMap *map_a, const CUtensorMap 
     for (int iter = 0; sched.get(iter, t) && !sh.abort_flag; ++iter) {
       const int acc = iter & 1;
       const uint32_t acc_phase = (iter >> 1) & 1u;
+      __nv_bfloat16 *rows[8];
+      gemm::find_rows(t, epi, int(rank) * BM + quarter * 32, lane, rows);   // my rows inside the pair's tile
       if (!sm100::mbar_wait(&sh.tmem_full[acc], acc_phase, &sh.abort_flag, WAIT_BUDGET_NS)) break;
       sm100::tcgen05_fence_after();
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * BN;
-      const int row_base = int(rank) * BM;   // my rows inside the pair's tile
       constexpr int OUT_CHUNKS = (SWIGLU ? BN / 2 : BN) / EPI_COLS;
 #pragma unroll 1
       for (int c = 0; c < OUT_CHUNKS; ++c) {
@@ -226,7 +227,7 @@ __device__ __forceinline__ void run(const CUtensorMap *map_a, const CUtensorMap 
           }
         }
         __syncwarp();
-        gemm::write_out_block<false>(t, epi, stg, row_base + quarter * 32, c * EPI_COLS, lane);
+        gemm::write_out_block<false>(t, rows, stg, c * EPI_COLS, lane);
         __syncwarp();
       }
       sm100::tcgen05_fence_before();

@@ -83,17 +83,16 @@ struct GatherSrc {
 };
 
 // Write-out of one warp's staged 32 x 64 bf16 block (padded rows in shared memory), 8 lanes per row, shared by the
-// one-CTA and the two-CTA cores.
-template <bool EPI_ADD, class Epilogue>
-__device__ __forceinline__ void write_out_block(const Tile &t, Epilogue &epi, const unsigned char *stg, int row0,
+// one-CTA and the two-CTA cores. `rows` are the eight rows that this lane writes (nullptr: none), looked up once a tile.
+template <bool EPI_ADD>
+__device__ __forceinline__ void write_out_block(const Tile &t, __nv_bfloat16 *const (&rows)[8], const unsigned char *stg,
                                                 int col0, int lane) {
 #pragma unroll
   for (int it = 0; it < 8; ++it) {
     const int r = it * 4 + lane / 8, seg = lane % 8;
-    const int row = row0 + r, col = col0 + seg * 8;
-    if (row >= t.rows || col >= t.cols) continue;
-    __nv_bfloat16 *out = epi.row_ptr(t, row);
-    if (out == nullptr) continue;
+    const int col = col0 + seg * 8;
+    __nv_bfloat16 *out = rows[it];
+    if (out == nullptr || col >= t.cols) continue;
     const unsigned char *src = stg + r * EPI_ROW_BYTES + seg * 16;
     __nv_bfloat16 *dst = out + col;
     if (col + 8 <= t.cols && (reinterpret_cast<uintptr_t>(dst) & 15u) == 0) {
@@ -110,6 +109,15 @@ __device__ __forceinline__ void write_out_block(const Tile &t, Epilogue &epi, co
   }
 }
 
+template <class Epilogue>
+__device__ __forceinline__ void find_rows(const Tile &t, Epilogue &epi, int row0, int lane, __nv_bfloat16 *(&rows)[8]) {
+#pragma unroll
+  for (int it = 0; it < 8; ++it) {
+    const int row = row0 + it * 4 + lane / 8;
+    rows[it] = row < t.rows ? epi.row_ptr(t, row) : nullptr;
+  }
+}
+
 struct Shared {
   uint64_t full[STAGES];
   uint64_t empty[STAGES];
@@ -119,7 +127,17 @@ struct Shared {
   volatile int abort_flag;
 };
 
-__device__ __forceinline__ float silu(float x) { return x / (1.0f + __expf(-x)); }
+// x / (1 + exp(-x)) without the branches of the IEEE division: the approximate reciprocal, and one Newton correction of
+// the quotient (the remainder x - d q is exact up to one rounding), which leaves at most the last bit. Where the correction
+// would meet inf * 0 (d past the reciprocal's range, x infinite) the uncorrected quotient is the answer: -0, inf or NaN.
+// With the IEEE form the block-scaled gate/up GEMM (16 experts, 7168 -> 2 x 2048) took 518 us for 1024 rows an expert and 117
+// for 64, with this one 505 and 107; the bf16 one for 64 rows 186 and 171.
+__device__ __forceinline__ float silu(float x) {
+  const float d = 1.0f + __expf(-x);
+  const float r = __fdividef(1.0f, d), q = x * r;
+  const float better = fmaf(fmaf(-d, q, x), r, q);
+  return d < 8e37f && x < 3e38f ? better : q;
+}
 
 // Scheduler: struct with  __device__ bool get(int iter, Tile &t)  (false: no more tiles for this CTA),
 //                         __device__ bool ready(const Tile &t)    (producer-side hook, bounded; false aborts)
@@ -274,6 +292,8 @@ __device__ __forceinline__ void run(const CUtensorMap *map_a, const CUtensorMap 
     for (int iter = 0; sched.get(iter, t) && !sh.abort_flag; ++iter) {
       const int acc = iter & 1;
       const uint32_t acc_phase = (iter >> 1) & 1u;
+      __nv_bfloat16 *rows[8];
+      find_rows(t, epi, quarter * 32, lane, rows);
       if (!sm100::mbar_wait(&sh.tmem_full[acc], acc_phase, &sh.abort_flag, WAIT_BUDGET_NS)) break;
       sm100::tcgen05_fence_after();
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * BN;
@@ -313,7 +333,7 @@ __device__ __forceinline__ void run(const CUtensorMap *map_a, const CUtensorMap 
           }
         }
         __syncwarp();
-        write_out_block<EPI_ADD>(t, epi, stg, quarter * 32, c * EPI_COLS, lane);
+        write_out_block<EPI_ADD>(t, rows, stg, c * EPI_COLS, lane);
         __syncwarp();
       }
       sm100::tcgen05_fence_before();

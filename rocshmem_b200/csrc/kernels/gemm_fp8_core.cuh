@@ -219,22 +219,18 @@ __device__ __forceinline__ void run(const CUtensorMap *map_a, const CUtensorMap 
       const size_t a_scale_row = A_GATHER ? static_cast<size_t>(gather->row_index[t.a_row + (row_ok ? row : 0)])
                                           : static_cast<size_t>(t.a_row + (row_ok ? row : 0));
       const float4 *sa4 = reinterpret_cast<const float4 *>((A_GATHER ? gather->scales : a_scale) + a_scale_row * k_blocks);
-      const float4 *sb4 = reinterpret_cast<const float4 *>(b_scale + static_cast<size_t>(t.b_row[SWIGLU ? 0 : half] / 128) * k_blocks);
-      const float4 *su4 = reinterpret_cast<const float4 *>(b_scale + static_cast<size_t>(t.b_row[1] / 128) * k_blocks);
+      // B's scales are the same for the whole warp, and one line holds 32 of them: they are read K block by K block, one
+      // ahead (four ahead like A's, they cost the registers that made the SwiGLU kernels spill).
+      const float *sb = b_scale + static_cast<size_t>(t.b_row[SWIGLU ? 0 : half] / 128) * k_blocks;
+      const float *su = b_scale + static_cast<size_t>(t.b_row[1] / 128) * k_blocks;
       // LATE_A: the A scales of a tile may still be on their way from another GPU until the producer has
       // seen the tile's rows arrive; the first finished K block proves it has. Read past L1 (__ldcg).
       if (LATE_A && !sm100::mbar_wait(&sh.tmem_full[buf], buf_phase, &sh.abort_flag, WAIT_BUDGET_NS)) break;
-      float4 a_next = __ldcg(sa4), b_next = sb4[0], u_next = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (SWIGLU) u_next = su4[0];
+      float4 a_next = __ldcg(sa4);
+      float b_next = sb[0], u_next = SWIGLU ? su[0] : 0.f;
       for (int kb4 = 0; kb4 < k_blocks / 4 && !sh.abort_flag; ++kb4) {
-        const float4 a_cur = a_next, b_cur = b_next, u_cur = u_next;
-        if (kb4 + 1 < k_blocks / 4) {  // fetched one group ahead of its use
-          a_next = __ldcg(sa4 + kb4 + 1);
-          b_next = sb4[kb4 + 1];
-          if (SWIGLU) u_next = su4[kb4 + 1];
-        }
-        const float scale[4] = {a_cur.x * b_cur.x, a_cur.y * b_cur.y, a_cur.z * b_cur.z, a_cur.w * b_cur.w};
-        const float scale_u[4] = {a_cur.x * u_cur.x, a_cur.y * u_cur.y, a_cur.z * u_cur.z, a_cur.w * u_cur.w};
+        const float4 a_cur = a_next;
+        if (kb4 + 1 < k_blocks / 4) a_next = __ldcg(sa4 + kb4 + 1);  // fetched one group ahead of its use
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           if (!sm100::mbar_wait(&sh.tmem_full[buf], buf_phase, &sh.abort_flag, WAIT_BUDGET_NS)) break;
@@ -243,8 +239,13 @@ __device__ __forceinline__ void run(const CUtensorMap *map_a, const CUtensorMap 
           // SwiGLU: the first half of the thread's columns are gate columns, the second half the matching up columns.
           const uint32_t col0 = SWIGLU ? half * 64 : half * 128;
           const uint32_t col2 = SWIGLU ? 128 + half * 64 : half * 128 + 64;
-          const unsigned long long s2 = sm100::pack_f32x2(scale[j], scale[j]);
-          const unsigned long long u2 = SWIGLU ? sm100::pack_f32x2(scale_u[j], scale_u[j]) : s2;
+          const float a_now = j == 0 ? a_cur.x : j == 1 ? a_cur.y : j == 2 ? a_cur.z : a_cur.w;
+          const unsigned long long s2 = sm100::pack_f32x2(a_now * b_next, a_now * b_next);
+          const unsigned long long u2 = SWIGLU ? sm100::pack_f32x2(a_now * u_next, a_now * u_next) : s2;
+          if (j < 3 || kb4 + 1 < k_blocks / 4) {
+            b_next = sb[kb4 * 4 + j + 1];
+            if (SWIGLU) u_next = su[kb4 * 4 + j + 1];
+          }
           uint32_t v[64];
           sm100::tmem_ld_32x64(tbuf + col0, v);
           sm100::tmem_ld_wait_for(v);
@@ -324,6 +325,13 @@ __device__ __forceinline__ void run(const CUtensorMap *map_a, const CUtensorMap 
         }
         __syncwarp();
       } else {
+      // The four rows that this lane writes, looked up once (a scatter reads each from an index).
+      __nv_bfloat16 *row_out[4];
+#pragma unroll
+      for (int it = 0; it < 4; ++it) {
+        const int orow = quarter * 32 + it * 8 + lane / 4;
+        row_out[it] = orow < t.rows ? epi.row_ptr(t, orow) : nullptr;
+      }
       // Write-out through the warp's padded staging rows, 32 columns at a time: 4 lanes per row write 64
       // contiguous bytes, 8 rows per instruction (instead of one row per thread in 16-byte pieces).
 #pragma unroll
@@ -340,10 +348,9 @@ __device__ __forceinline__ void run(const CUtensorMap *map_a, const CUtensorMap 
 #pragma unroll
         for (int it = 0; it < 4; ++it) {
           const int r = it * 8 + lane / 4, seg = lane % 4;
-          const int orow = quarter * 32 + r;
           const int col = col0 + c * 32 + seg * 8;
-          if (orow < t.rows && col < t.cols) {
-            __nv_bfloat16 *out = epi.row_ptr(t, orow);
+          if (col < t.cols) {
+            __nv_bfloat16 *out = row_out[it];
             if (out != nullptr) {
               const unsigned char *src = stg + r * EPI_ROW_BYTES + seg * 16;
               __nv_bfloat16 *dst = out + col;
