@@ -84,11 +84,13 @@ void bind_gemm(py::module_ &m) {
         py::arg("keep") = 0);
   m.def("ag_gemm_fp8", [](uintptr_t team, uintptr_t x_q, uintptr_t x_s, uintptr_t gq, uintptr_t gs, uintptr_t flags,
                           uintptr_t b_q, uintptr_t b_s, uintptr_t c, int m_shard, int N, int K, unsigned epoch,
-                          int swiglu, uintptr_t stream) {
+                          int swiglu, uintptr_t stream, uintptr_t c_q, uintptr_t c_s) {
     check(ag_gemm_fp8(reinterpret_cast<rocshmem_team_t>(team), P<void>(x_q), P<float>(x_s), P<void>(gq), P<float>(gs),
                       P<unsigned long long>(flags), P<void>(b_q), P<float>(b_s), P<void>(c), m_shard, N, K, epoch,
-                      swiglu, P<void>(stream)), "ag_gemm_fp8");
-  });
+                      swiglu, P<void>(stream), P<void>(c_q), P<float>(c_s)), "ag_gemm_fp8");
+  }, py::arg("team"), py::arg("x_q"), py::arg("x_s"), py::arg("gathered_q"), py::arg("gathered_s"), py::arg("flags"),
+        py::arg("b_q"), py::arg("b_s"), py::arg("c"), py::arg("m_shard"), py::arg("N"), py::arg("K"), py::arg("epoch"),
+        py::arg("swiglu"), py::arg("stream"), py::arg("c_q") = 0, py::arg("c_s") = 0);
   m.def("gemm_rs_fp8", [](uintptr_t team, uintptr_t a_q, uintptr_t a_s, uintptr_t b_q, uintptr_t b_s,
                           uintptr_t staging, uintptr_t out, int m_shard, int N, int K, uintptr_t counter,
                           unsigned epoch, uintptr_t stream) {

@@ -96,7 +96,9 @@ int gemm_rs_bf16(rocshmem_team_t team, const void *a, const void *b, void *stagi
 // [N / 128, K / 128]. K must be a multiple of 512, N of 128 (256 with swiglu).
 int ag_gemm_fp8(rocshmem_team_t team, const void *x_q, const float *x_s, void *gathered_q, float *gathered_s,
                 unsigned long long *flags, const void *b_q, const float *b_scale, void *c, int m_shard, int n, int k,
-                unsigned epoch, int swiglu, void *stream);
+                unsigned epoch, int swiglu, void *stream, void *c_q = nullptr, float *c_s = nullptr);
+// With c_q (and swiglu) the result is not stored in c but quantised: c_q [n_ranks * m_shard, n / 2] e4m3 and
+// c_s [n_ranks * m_shard, n / 256].
 int gemm_rs_fp8(rocshmem_team_t team, const void *a_q, const float *a_scale, const void *b_q, const float *b_scale,
                 void *staging, void *out, int m_shard, int n, int k, unsigned long long *grid_counter, unsigned epoch,
                 void *stream);

@@ -72,8 +72,8 @@ class TensorParallelMLP:
 
 class TensorParallelMLPFp8:
     """The same block with block-scaled e4m3 GEMMs: activations are quantised 1 x 128 (the input shard before
-    the all-gather, the hidden activation before the down projection), weights 128 x 128. Four kernels per
-    forward: quantise, all-gather -> GEMM -> SwiGLU, quantise, GEMM -> reduce-scatter."""
+    the all-gather, the hidden activation in the first GEMM's epilogue), weights 128 x 128. Three kernels per
+    forward: quantise, all-gather -> GEMM -> SwiGLU -> quantise, GEMM -> reduce-scatter."""
 
     def __init__(self, d_model: int, d_ff: int, m_shard: int, team: Optional[rt.Team] = None, seed: int = 0):
         self.tp = gemm.TensorParallelLinearFp8(m_shard, team=team)
@@ -96,11 +96,9 @@ class TensorParallelMLPFp8:
 
     @traced("rocshmem_b200.tp_mlp_fp8")
     def forward(self, x_shard: torch.Tensor, out: Optional[torch.Tensor] = None, stream=None) -> torch.Tensor:
-        """Quantise the shard, all-gather -> up projection with SwiGLU, quantise, down projection -> reduce-scatter."""
+        """Quantise the shard, all-gather -> up projection with SwiGLU, quantised; down projection -> reduce-scatter."""
         self.tp.set_input(x_shard, stream)
-        self.tp.ag_gemm(self.w1_q, self.w1_s, out=self.h, swiglu=True, stream=stream)
-        gemm.quantize_1x128_into(self.h, self.h_q, self.h_s, stream)
-        self.tp.kernel_launches += 1
+        self.tp.ag_gemm_quantized(self.w1_q, self.w1_s, self.h_q, self.h_s, stream=stream)
         return self.tp.gemm_rs(self.h_q, self.h_s, self.w2_q, self.w2_s, out=out, stream=stream)
 
     __call__ = forward

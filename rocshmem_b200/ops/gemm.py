@@ -382,6 +382,21 @@ class TensorParallelLinearFp8:
         self.kernel_launches += 1
         return out
 
+    def ag_gemm_quantized(self, w_q: torch.Tensor, w_s: torch.Tensor, out_q: torch.Tensor, out_s: torch.Tensor,
+                          stream=None) -> None:
+        """:meth:`ag_gemm` with SwiGLU whose result leaves the kernel as the next GEMM's operand: ``out_q [n_ranks *
+        m_shard, N / 2]`` e4m3 with one fp32 scale per 128 columns in ``out_s [n_ranks * m_shard, N / 256]``."""
+        N, K = w_q.shape
+        _check8(out_q, out_s, "out")
+        if tuple(out_q.shape) != (self.n_ranks * self.m_shard, N // 2) or tuple(out_s.shape) != (out_q.shape[0], N // 256):
+            raise ValueError("ag_gemm_quantized: out shapes")
+        x_q, x_s, g_q, g_s, flags, _ = buf = self._ag_buffers(K)
+        buf[5] += 1
+        rt._C().ag_gemm_fp8(self.team.handle, x_q.data_ptr(), x_s.data_ptr(), g_q.data_ptr(), g_s.data_ptr(),
+                            flags.data_ptr(), w_q.data_ptr(), w_s.data_ptr(), 0, self.m_shard, N, K, buf[5], 1,
+                            _stream(stream), out_q.data_ptr(), out_s.data_ptr())
+        self.kernel_launches += 1
+
     def gemm_rs(self, a_q: torch.Tensor, a_s: torch.Tensor, w_q: torch.Tensor, w_s: torch.Tensor,
                 out: Optional[torch.Tensor] = None, stream=None) -> torch.Tensor:
         """``a @ w.T`` (block-scaled e4m3) fused with the reduce-scatter of the bf16 result over the team."""
