@@ -69,9 +69,65 @@ __device__ __forceinline__ typename Acc<T>::type combine(typename Acc<T>::type a
   }
 }
 
+// The vectors of reduce_range for teams of at most B members: every thread has the loads of U vectors of all members in
+// flight before it uses the first of them. `base` is the first element; vectors tid, tid + nthr, ... of `nvec` are taken.
+//
+// The pass is bound by the bytes in flight: one block of 512 threads a SM, so B * U = 16 loads of 16 bytes a thread are
+// 128 KiB a SM (64 of a thread's 128 registers).
+// Four PEs on one GPU, 16 Mi bf16 elements: 65.9 us with eight loads, 55.1 with sixteen (4.9 TB/s).
+template <typename T, int OP, bool ALL, int B, int U>
+__device__ __forceinline__ void reduce_vectors(const rocshmem_team_dev *t, T *dest, const T *source, size_t base,
+                                               size_t nvec, size_t tid, size_t nthr, int op) {
+  using A = typename Acc<T>::type;
+  constexpr int VEC = 16 / sizeof(T);
+  const int n = t->size;
+  for (size_t v = tid; v < nvec; v += U * nthr) {
+    int4 raw[U][B];
+#pragma unroll
+    for (int k = 0; k < B; ++k) {
+      if (k < n) {
+        // Start with my own copy, then the peers in rotated order so that at any moment the
+        // members read from different sources.
+        const T *from = remote_ptr(source, team_pe_to_world(t, (t->my_pe + k) % n));
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          if (v + u * nthr < nvec) raw[u][k] = ld_global_16(from + base + (v + u * nthr) * VEC);
+        }
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (v + u * nthr < nvec) {
+        A acc[VEC];
+#pragma unroll
+        for (int k = 0; k < B; ++k) {
+          if (k < n) {
+            const T *x = reinterpret_cast<const T *>(&raw[u][k]);
+#pragma unroll
+            for (int q = 0; q < VEC; ++q) acc[q] = k == 0 ? to_acc<T>(x[q]) : combine<T, OP>(acc[q], to_acc<T>(x[q]), op);
+          }
+        }
+        int4 out;
+        T *o = reinterpret_cast<T *>(&out);
+#pragma unroll
+        for (int q = 0; q < VEC; ++q) o[q] = from_acc<T>(acc[q]);
+        const size_t e = base + (v + u * nthr) * VEC;
+        if (ALL) {
+          for (int d = 0; d < n; ++d) {
+            st_global_16(remote_ptr(dest + e, team_pe_to_world(t, (t->my_pe + d) % n)), out);
+          }
+        } else {
+          st_global_16(dest + e, out);
+        }
+      }
+    }
+  }
+}
+
 // Reduce elements [lo, hi) over all members; the result goes to the local dest only (ALL == false)
 // or to every member's dest (ALL == true). `tid`/`nthr` enumerate the threads working on the range.
-template <typename T, int OP, bool ALL>
+// SMALL: the team has at most four members.
+template <typename T, int OP, bool ALL, bool SMALL>
 __device__ __forceinline__ void reduce_range(const rocshmem_team_dev *t, T *dest, const T *source,
                                              size_t lo, size_t hi, size_t tid, size_t nthr, int op,
                                              bool aligned) {
@@ -81,71 +137,75 @@ __device__ __forceinline__ void reduce_range(const rocshmem_team_dev *t, T *dest
   size_t scalar_from = lo;
   if (aligned && (lo % VEC) == 0) {
     const size_t nvec = (hi - lo) / VEC;
-    // Two vectors per thread and pass; the loads of both (one per member, up to 8 members at a
-    // time) are issued before any value is used.
-    constexpr int U = 2;
-    for (size_t v = tid; v < nvec; v += U * nthr) {
-      size_t e[U];
-      bool live[U];
+    if constexpr (SMALL) {
+      reduce_vectors<T, OP, ALL, 4, 4>(t, dest, source, lo, nvec, tid, nthr, op);
+    } else {
+      // Two vectors per thread and pass; the loads of both (one per member, up to 8 members at a
+      // time) are issued before any value is used.
+      constexpr int U = 2;
+      for (size_t v = tid; v < nvec; v += U * nthr) {
+        size_t e[U];
+        bool live[U];
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        live[u] = v + u * nthr < nvec;
-        e[u] = lo + (v + u * nthr) * VEC;
-      }
-      int4 raw[U][8];
-      A acc[U][VEC];
-      int done = 0;
-      bool first = true;
-      while (done < n) {
-        const int batch = (n - done) < 8 ? (n - done) : 8;
+        for (int u = 0; u < U; ++u) {
+          live[u] = v + u * nthr < nvec;
+          e[u] = lo + (v + u * nthr) * VEC;
+        }
+        int4 raw[U][8];
+        A acc[U][VEC];
+        int done = 0;
+        bool first = true;
+        while (done < n) {
+          const int batch = (n - done) < 8 ? (n - done) : 8;
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          if (k < batch) {
-            // Start with my own copy, then the peers in rotated order so that at any moment the
-            // members read from different sources.
-            const int j = (t->my_pe + done + k) % n;
-            const int w = team_pe_to_world(t, j);
+          for (int k = 0; k < 8; ++k) {
+            if (k < batch) {
+              // Start with my own copy, then the peers in rotated order so that at any moment the
+              // members read from different sources.
+              const int j = (t->my_pe + done + k) % n;
+              const int w = team_pe_to_world(t, j);
 #pragma unroll
-            for (int u = 0; u < U; ++u) {
-              if (live[u]) raw[u][k] = ld_global_16(remote_ptr(source + e[u], w));
+              for (int u = 0; u < U; ++u) {
+                if (live[u]) raw[u][k] = ld_global_16(remote_ptr(source + e[u], w));
+              }
             }
           }
-        }
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          if (k < batch) {
+          for (int k = 0; k < 8; ++k) {
+            if (k < batch) {
 #pragma unroll
-            for (int u = 0; u < U; ++u) {
-              if (live[u]) {
-                const T *x = reinterpret_cast<const T *>(&raw[u][k]);
-                if (first && k == 0) {
+              for (int u = 0; u < U; ++u) {
+                if (live[u]) {
+                  const T *x = reinterpret_cast<const T *>(&raw[u][k]);
+                  if (first && k == 0) {
 #pragma unroll
-                  for (int q = 0; q < VEC; ++q) acc[u][q] = to_acc<T>(x[q]);
-                } else {
+                    for (int q = 0; q < VEC; ++q) acc[u][q] = to_acc<T>(x[q]);
+                  } else {
 #pragma unroll
-                  for (int q = 0; q < VEC; ++q) acc[u][q] = combine<T, OP>(acc[u][q], to_acc<T>(x[q]), op);
+                    for (int q = 0; q < VEC; ++q) acc[u][q] = combine<T, OP>(acc[u][q], to_acc<T>(x[q]), op);
+                  }
                 }
               }
             }
           }
+          first = false;
+          done += batch;
         }
-        first = false;
-        done += batch;
-      }
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        if (!live[u]) continue;
-        int4 out;
-        T *o = reinterpret_cast<T *>(&out);
+        for (int u = 0; u < U; ++u) {
+          if (!live[u]) continue;
+          int4 out;
+          T *o = reinterpret_cast<T *>(&out);
 #pragma unroll
-        for (int q = 0; q < VEC; ++q) o[q] = from_acc<T>(acc[u][q]);
-        if (ALL) {
-          for (int d = 0; d < n; ++d) {
-            const int j = (t->my_pe + d) % n;
-            st_global_16(remote_ptr(dest + e[u], team_pe_to_world(t, j)), out);
+          for (int q = 0; q < VEC; ++q) o[q] = from_acc<T>(acc[u][q]);
+          if (ALL) {
+            for (int d = 0; d < n; ++d) {
+              const int j = (t->my_pe + d) % n;
+              st_global_16(remote_ptr(dest + e[u], team_pe_to_world(t, j)), out);
+            }
+          } else {
+            st_global_16(dest + e[u], out);
           }
-        } else {
-          st_global_16(dest + e[u], out);
         }
       }
     }
@@ -173,7 +233,7 @@ __global__ void __launch_bounds__(64) barrier_kernel(rocshmem_team_t team) {
   detail::team_barrier(const_cast<rocshmem_team_dev *>(t), false);
 }
 
-template <typename T, int OP>
+template <typename T, int OP, bool SMALL>
 __global__ void __launch_bounds__(kThreads)
 allreduce_one_shot_kernel(rocshmem_team_t team, T *dest_arg, const T *source_arg, size_t nelems, int op) {
   const rocshmem_team_dev *t = detail::team_of(team);
@@ -182,14 +242,14 @@ allreduce_one_shot_kernel(rocshmem_team_t team, T *dest_arg, const T *source_arg
   const T *source = detail::local_ptr(const_cast<T *>(source_arg));
   const bool aligned = ((reinterpret_cast<uintptr_t>(dest) | reinterpret_cast<uintptr_t>(source)) & 15u) == 0;
   if (!block_pair_barrier(t, blockIdx.x)) return;
-  reduce_range<T, OP, false>(t, dest, source, 0, nelems, size_t(blockIdx.x) * blockDim.x + threadIdx.x,
+  reduce_range<T, OP, false, SMALL>(t, dest, source, 0, nelems, size_t(blockIdx.x) * blockDim.x + threadIdx.x,
                              size_t(gridDim.x) * blockDim.x, op, aligned);
   // Nobody overwrites a source while a peer may still be reading it. The result is local, nothing is
   // handed over, so the relaxed form of the barrier is enough.
   block_pair_barrier(t, blockIdx.x, false);
 }
 
-template <typename T, int OP>
+template <typename T, int OP, bool SMALL>
 __global__ void __launch_bounds__(kThreads)
 allreduce_two_shot_kernel(rocshmem_team_t team, T *dest_arg, const T *source_arg, size_t nelems, int op) {
   const rocshmem_team_dev *t = detail::team_of(team);
@@ -204,7 +264,7 @@ allreduce_two_shot_kernel(rocshmem_team_t team, T *dest_arg, const T *source_arg
   if (lo > nelems) lo = nelems;
   if (hi > nelems) hi = nelems;
   if (!block_pair_barrier(t, blockIdx.x)) return;
-  reduce_range<T, OP, true>(t, dest, source, lo, hi, size_t(blockIdx.x) * blockDim.x + threadIdx.x,
+  reduce_range<T, OP, true, SMALL>(t, dest, source, lo, hi, size_t(blockIdx.x) * blockDim.x + threadIdx.x,
                             size_t(gridDim.x) * blockDim.x, op, aligned);
   block_pair_barrier(t, blockIdx.x);
 }
@@ -590,12 +650,15 @@ int launch_allreduce_typed(rocshmem_team_t team, void *dest, const void *source,
       return launch_pes(k, clamp_blocks(k, want), kThreads, 0, stream, false, team, d, s, nelems);
     }
   }
-  const bool sum = op == ROCSHMEM_SUM;
+  // Small teams have a kernel of their own: both loops in one made it long enough to cost small payloads 2 us.
+  const bool sum = op == ROCSHMEM_SUM, small = n <= 4;
   if (algo == ALLREDUCE_ONE_SHOT) {
-    auto k = sum ? allreduce_one_shot_kernel<T, ROCSHMEM_SUM> : allreduce_one_shot_kernel<T, OP_RUNTIME>;
+    auto k = small ? (sum ? allreduce_one_shot_kernel<T, ROCSHMEM_SUM, true> : allreduce_one_shot_kernel<T, OP_RUNTIME, true>)
+                 : (sum ? allreduce_one_shot_kernel<T, ROCSHMEM_SUM, false> : allreduce_one_shot_kernel<T, OP_RUNTIME, false>);
     return launch_pes(k, clamp_blocks(k, want), kThreads, 0, stream, false, team, d, s, nelems, op);
   }
-  auto k = sum ? allreduce_two_shot_kernel<T, ROCSHMEM_SUM> : allreduce_two_shot_kernel<T, OP_RUNTIME>;
+  auto k = small ? (sum ? allreduce_two_shot_kernel<T, ROCSHMEM_SUM, true> : allreduce_two_shot_kernel<T, OP_RUNTIME, true>)
+                 : (sum ? allreduce_two_shot_kernel<T, ROCSHMEM_SUM, false> : allreduce_two_shot_kernel<T, OP_RUNTIME, false>);
   return launch_pes(k, clamp_blocks(k, want), kThreads, 0, stream, false, team, d, s, nelems, op);
 }
 
@@ -626,10 +689,14 @@ void load_allreduce_now(int *rc) {
     load_now(allreduce_ll_kernel<T, ROCSHMEM_SUM>, rc);
     load_now(allreduce_ll_kernel<T, OP_RUNTIME>, rc);
   }
-  load_now(allreduce_one_shot_kernel<T, ROCSHMEM_SUM>, rc);
-  load_now(allreduce_one_shot_kernel<T, OP_RUNTIME>, rc);
-  load_now(allreduce_two_shot_kernel<T, ROCSHMEM_SUM>, rc);
-  load_now(allreduce_two_shot_kernel<T, OP_RUNTIME>, rc);
+  load_now(allreduce_one_shot_kernel<T, ROCSHMEM_SUM, true>, rc);
+  load_now(allreduce_one_shot_kernel<T, ROCSHMEM_SUM, false>, rc);
+  load_now(allreduce_one_shot_kernel<T, OP_RUNTIME, true>, rc);
+  load_now(allreduce_one_shot_kernel<T, OP_RUNTIME, false>, rc);
+  load_now(allreduce_two_shot_kernel<T, ROCSHMEM_SUM, true>, rc);
+  load_now(allreduce_two_shot_kernel<T, ROCSHMEM_SUM, false>, rc);
+  load_now(allreduce_two_shot_kernel<T, OP_RUNTIME, true>, rc);
+  load_now(allreduce_two_shot_kernel<T, OP_RUNTIME, false>, rc);
 }
 }  // namespace
 
