@@ -84,6 +84,7 @@ struct DispatchArgs {
   int num_tokens;
   unsigned epoch;
   rocshmem_team_t team;
+  void *zero_y;   // low-latency mode, team of one: result rows to clear as their tokens get them; nullptr: none
 };
 
 __device__ __forceinline__ float group8_max(float v) {
@@ -753,6 +754,10 @@ __global__ void __launch_bounds__(kLlThreads) ep_ll_dispatch_kernel(DispatchArgs
       sent_slot[size_t(tok) * P + tid] = slot;
     }
     __syncthreads();
+    if (a.zero_y != nullptr && s_slot[0] >= 0) {
+      int4 *y = reinterpret_cast<int4 *>(static_cast<__nv_bfloat16 *>(rebase(a.zero_y)) + size_t(s_slot[0]) * H);
+      for (unsigned v = tid; v < unsigned(H / 8); v += nthr) y[v] = make_int4(0, 0, 0, 0);
+    }
     if (a.cfg.quantize) {
 #pragma unroll
       for (int m = 0; m < kMine; ++m) {
@@ -1106,13 +1111,14 @@ unsigned long long ep_combine_fetches(const EpConfig &cfg, int num_tokens) {
 }
 
 int ep_dispatch(rocshmem_team_t team, const EpConfig &cfg, const EpBuffers &buf, const void *x,
-                const int *topk_idx, const float *topk_w, int num_tokens, unsigned epoch, void *stream) {
+                const int *topk_idx, const float *topk_w, int num_tokens, unsigned epoch, void *stream, void *zero_y) {
   Runtime &rt = Runtime::instance();
   HostTeam *ht = rt.team_from_handle(team);
   if (!ht) return cudaErrorInvalidValue;
   if (int rc = validate(cfg, ht->world.size, num_tokens)) return rc;
   if (cfg.expert_layout && (!buf.lay_offsets || !buf.lay_row || !buf.lay_k || !buf.lay_w)) return cudaErrorInvalidValue;
-  DispatchArgs a{cfg, buf, static_cast<const __nv_bfloat16 *>(x), topk_idx, topk_w, num_tokens, epoch, team};
+  DispatchArgs a{cfg, buf, static_cast<const __nv_bfloat16 *>(x), topk_idx, topk_w, num_tokens, epoch, team, zero_y};
+  if (zero_y != nullptr && (!cfg.low_latency || ht->world.size != 1)) return cudaErrorInvalidValue;
   if (cfg.low_latency) {
     if (buf.work_counter == nullptr) return cudaErrorInvalidValue;
     // A block per token; with several PEs per process the launch is cooperative and must fit the GPU at once.

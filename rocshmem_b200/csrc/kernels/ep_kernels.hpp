@@ -111,8 +111,9 @@ struct EpBuffers {
 
 // x [T, hidden] bf16, topk_idx [T, top_k] int32 (global expert ids, -1 = unused), topk_w [T, top_k] fp32.
 // `epoch` must increase by one per dispatch call on these buffers (the same value on every member).
+// zero_y (low-latency mode, team of one): a result buffer whose rows are cleared as tokens get them.
 int ep_dispatch(rocshmem_team_t team, const EpConfig &cfg, const EpBuffers &buf, const void *x,
-                const int *topk_idx, const float *topk_w, int num_tokens, unsigned epoch, void *stream);
+                const int *topk_idx, const float *topk_w, int num_tokens, unsigned epoch, void *stream, void *zero_y = nullptr);
 
 // y: symmetric [P * max_tokens, hidden] bf16 in the row layout produced by dispatch. out [T, hidden]
 // bf16 (local). Every token receives the sum over the ranks it was sent to of that rank's row,

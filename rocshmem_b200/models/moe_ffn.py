@@ -114,24 +114,30 @@ class MoEFeedForward:
                 marks.append((name, ev))
 
         mark("start")
-        d.dispatch(x, topk_idx, topk_weights, stream=stream)
+        # The down projection adds into the result rows, which therefore start from zero. In low-latency mode a rank on
+        # its own clears them in the dispatch kernel; otherwise that runs on a side stream beside the first GEMM (its
+        # launch and the events are host time that a small decode step cannot hide: 44 tokens, 8 experts of 2048 x 1024:
+        # 67 us a call with them, 59 without).
+        cleared = d.low_latency and self.n_ranks == 1
+        d.dispatch(x, topk_idx, topk_weights, stream=stream, zero_result=cleared)
         mark("dispatch")
         offsets, lay_row, _, lay_w = d.expert_pairs()
         y = d.result_buffer()
-        # The down projection adds into the result rows, which therefore start from zero; clearing them runs on a
-        # side stream beside the first GEMM.
-        self.ev_dispatched.record(cur)
-        self.side.wait_event(self.ev_dispatched)
-        C.moe_zero_rows(d.recv_info.data_ptr(), self.n_ranks, self.hidden, y.data_ptr(), self.side.cuda_stream)
-        self.ev_zeroed.record(self.side)
-        launches = 3
+        launches = 2
+        if not cleared:
+            self.ev_dispatched.record(cur)
+            self.side.wait_event(self.ev_dispatched)
+            C.moe_zero_rows(d.recv_info.data_ptr(), self.n_ranks, self.hidden, y.data_ptr(), self.side.cuda_stream)
+            self.ev_zeroed.record(self.side)
+            launches += 1
         if self.fp8_experts:
             # Received e4m3 rows and their scales feed the first GEMM as they are (gathered by its producer warps);
             # its epilogue quantises the hidden activation for the second one.
             gemm.grouped_gemm_fp8_swiglu_quant(d.recv_x, d.recv_scales, self.w13_q, self.w13_s, offsets, self.h_q,
                                                self.h_s, row_index=lay_row, stream=stream)
             mark("gemm_gate_up")
-            cur.wait_event(self.ev_zeroed)
+            if not cleared:
+                cur.wait_event(self.ev_zeroed)
             gemm.grouped_gemm_fp8_scatter_add(self.h_q, self.h_s, self.w2_q, self.w2_s, offsets, lay_row, y,
                                               weights=lay_w, stream=stream)
         else:
@@ -145,7 +151,8 @@ class MoEFeedForward:
                 gemm.grouped_gemm_bf16_gathered(d.recv_x, lay_row, self.w13, offsets, swiglu=True, out=self.h,
                                                 stream=stream)
             mark("gemm_gate_up")
-            cur.wait_event(self.ev_zeroed)
+            if not cleared:
+                cur.wait_event(self.ev_zeroed)
             gemm.grouped_gemm_bf16_scatter_add(self.h, self.w2, offsets, lay_row, y, weights=lay_w, stream=stream)
         mark("gemm_down")
         out = d.combine(y, topk_idx, topk_weights, x.shape[0], weighted=False, out=out, stream=stream)

@@ -186,9 +186,10 @@ class EpDispatcher:
 
     # -- operations -------------------------------------------------------------------------------------------
     def dispatch(self, x: torch.Tensor, topk_idx: torch.Tensor, topk_weights: torch.Tensor,
-                 stream=None) -> DispatchResult:
+                 stream=None, zero_result: bool = False) -> DispatchResult:
         """x [T, hidden] bf16, topk_idx [T, top_k] int32 (global expert ids, -1 unused), topk_weights
-        [T, top_k] fp32; all contiguous on this PE's GPU. Stream-ordered."""
+        [T, top_k] fp32; all contiguous on this PE's GPU. Stream-ordered. ``zero_result`` (low-latency mode, team of
+        one): the received rows' slots of :meth:`result_buffer` are cleared by the same kernel."""
         T = x.shape[0]
         if T > self.max_tokens or x.shape[1] != self.hidden or x.dtype != torch.bfloat16:
             raise ValueError("dispatch: x must be [T <= max_tokens, hidden] bf16")
@@ -200,7 +201,8 @@ class EpDispatcher:
             if not t.is_contiguous():
                 raise ValueError("dispatch: tensors must be contiguous")
         with trace_range("rocshmem_b200.ep_dispatch"):
-            self._h.dispatch(x.data_ptr(), topk_idx.data_ptr(), topk_weights.data_ptr(), T, _stream(stream))
+            self._h.dispatch(x.data_ptr(), topk_idx.data_ptr(), topk_weights.data_ptr(), T, _stream(stream),
+                             self.result_buffer().data_ptr() if zero_result else 0)
         self.kernel_launches += 1
         return self._result()
 

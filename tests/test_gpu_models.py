@@ -173,3 +173,26 @@ def test_dispatch_and_combine_of_a_rank_on_its_own(shm, T, H, K, quantize):
             clean(shm)
             assert (out.float() - want).abs().max().item() <= 2 ** -8 * want.abs().max().item()   # one bf16 rounding
     d.destroy()
+
+
+@pytest.mark.parametrize("quantize", [True, False])
+@pytest.mark.parametrize("T", [1, 37, 128])
+def test_moe_feed_forward_low_latency_alone(shm, quantize, T):
+    """Low-latency mode of a rank on its own: the dispatch kernel clears the result rows that the down projection adds
+    into, so a second call on the same layer is not added to the first."""
+    from rocshmem_b200.models import moe_ffn
+    from rocshmem_b200.ops import gemm, moe
+    E, K, H, I = 8, 3, 1024, 512
+    layer = moe_ffn.MoEFeedForward(E, K, H, I, max_tokens=128, seed=2, quantize=quantize, low_latency=True)
+    for rep in range(3):
+        x = torch.randn(T, H, generator=torch.Generator().manual_seed(T + rep)).to(torch.bfloat16)
+        idx, w = moe.make_routing(T, E, K, seed=T + rep)
+        if T > 1:
+            idx[rep, :] = -1                     # a token without an expert: its row is zero
+        want = moe_ffn.reference_forward(x, idx, w, H, I, seed=2, quantize=quantize, fp8_experts=quantize)
+        before = gemm.gemm_error_count()
+        out = layer(x.cuda(), idx.cuda(), w.cuda()).float().cpu()
+        clean(shm)
+        assert gemm.gemm_error_count() == before
+        assert (out - want).abs().max().item() <= 5e-2 * want.abs().max().item() + 0.05
+    layer.destroy()
