@@ -1,7 +1,7 @@
 """Expert-parallel MoE feed-forward layer (SwiGLU experts) built from this package's kernels.
 
 One call runs, stream-ordered and without a host synchronisation, as four kernels (plus a memset-like one on a
-side stream)::
+side stream, which the low-latency dispatch of a team of one replaces)::
 
     dispatch       fp8 1x128 rows over NVLink; its tail groups the received (row, k) pairs by local expert
     gate/up GEMM   grouped block-scaled e4m3 tcgen05 GEMM whose producer warps gather the received rows (and the
