@@ -34,6 +34,7 @@
 #include "gemm_core.cuh"
 #include "gemm2_core.cuh"
 #include "gemm_fp8_core.cuh"
+#include "fused_select.hpp"
 #include "gemm_kernels.hpp"
 #include "gemm_tmap.hpp"
 #include "launch.cuh"
@@ -566,10 +567,8 @@ int prepare_smem(K kernel) {
   return e == cudaSuccess ? 0 : static_cast<int>(e);
 }
 
-// Whether [a, a + a_bytes) and [b, b + b_bytes) share memory.
 bool overlaps(const void *a, size_t a_bytes, const void *b, size_t b_bytes) {
-  const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
-  return x < y + b_bytes && y < x + a_bytes;
+  return kernels::overlaps(Span{a, a_bytes}, Span{b, b_bytes});
 }
 
 int copy_aside(void *dst, const void *src, size_t bytes, void *stream) {
@@ -596,11 +595,17 @@ int ag_gemm_bf16(rocshmem_team_t team, const void *x_shard, void *gathered, unsi
   const bool alone = P == 1;
   if (keep != nullptr && !alone) return cudaErrorInvalidValue;
   if (alone) {
-    // The shard is read in place, unless the result would overwrite rows that are still to be read.
+    // The shard is read in place, unless something that the kernel writes shares memory with it.
     const size_t x_bytes = size_t(m_shard) * k * 2, c_bytes = size_t(m_shard) * (swiglu ? n / 2 : n) * 2;
-    if (overlaps(x_shard, x_bytes, c, c_bytes)) {
+    const AlonePlan plan = plan_alone(Span{x_shard, x_bytes}, Span{keep, keep != nullptr ? x_bytes : 0},
+                                      Span{b, size_t(n) * k * 2}, Span{c, c_bytes});
+    if (plan.rows_aside) {
       if (int rc = copy_aside(gathered, x_shard, x_bytes, stream)) return rc;
       x_shard = gathered;
+    }
+    if (plan.keep_first) {
+      if (int rc = copy_aside(keep, x_shard, x_bytes, stream)) return rc;
+      keep = nullptr;
     }
   }
   CUtensorMap map_a, map_b;

@@ -21,6 +21,7 @@
 #include "team.hpp"
 #include "../kernels/coll_select.hpp"
 #include "../kernels/ep_kernels.hpp"
+#include "../kernels/fused_select.hpp"
 
 using namespace rocshmem;
 
@@ -356,6 +357,73 @@ static void test_ep_config_limits() {
   EXPECT(ep_ll_combine_blocks(c) == ROCSHMEM_LIB_MAX_BLOCKS);
 }
 
+// all-gather -> GEMM on a team of one: what the plan does gives the buffers that the documented order gives (the rows become
+// the input buffer's content, then the result is written), wherever the operands lie. The "GEMM" of this model reads the
+// weight and the rows it is given when the kernel runs, and writes two result bytes; inside the kernel the reads, the copy
+// into the input buffer and the result come in every order that the hardware may take.
+static void test_fused_alone_plan() {
+  using namespace rocshmem::kernels;
+  constexpr int L = 4, MEM = 16, GATHER = 12;   // operands of four bytes anywhere in the first twelve
+  using Mem = std::vector<int>;
+  auto product = [](const Mem &m, int rows, int w) {
+    int s = 0;
+    for (int i = 0; i < L; ++i) s += (i + 1) * m[rows + i] * (m[w + i] + 3);
+    return s;
+  };
+  auto result = [](Mem &m, int c, int v) {
+    for (int i = 0; i < L; ++i) m[c + i] = v + i;
+  };
+  auto copy = [](Mem &m, int to, int from) {
+    Mem tmp(m.begin() + from, m.begin() + from + L);
+    for (int i = 0; i < L; ++i) m[to + i] = tmp[i];
+  };
+  char base[MEM];
+  for (int x = 0; x + L <= GATHER; ++x) {
+    for (int keep = 0; keep + L <= GATHER; ++keep) {
+      for (int w = 0; w + L <= GATHER; ++w) {
+        for (int c = 0; c + L <= GATHER; ++c) {
+          if (std::abs(w - c) < L) continue;   // a result over the weight was never ordered
+          Mem want(MEM);
+          for (int i = 0; i < MEM; ++i) want[i] = 7 * i + 1;
+          const Mem start = want;
+          copy(want, keep, x);
+          result(want, c, product(want, keep, w));
+          const AlonePlan plan = plan_alone(Span{base + x, L}, Span{base + keep, L}, Span{base + w, L}, Span{base + c, L});
+          for (int order = 0; order < 6; ++order) {
+            Mem m = start;
+            int rows = x, kept = keep;
+            if (plan.rows_aside) copy(m, GATHER, rows), rows = GATHER;
+            if (plan.keep_first) copy(m, keep, rows), kept = -1;
+            // read / copy / write of the kernel; the product cannot be written before it has been read, but the copy may
+            // come before, between or after, and half of it before and half after.
+            const Mem before = m;
+            int v = 0;
+            auto half = [&](int h) {
+              if (kept < 0) return;
+              for (int i = h * L / 2; i < (h + 1) * L / 2; ++i) m[kept + i] = m[rows + i];
+            };
+            if (order == 0) half(0), half(1), v = product(m, rows, w), result(m, c, v);
+            if (order == 1) v = product(m, rows, w), half(0), half(1), result(m, c, v);
+            if (order == 2) v = product(m, rows, w), result(m, c, v), half(0), half(1);
+            if (order == 3) half(0), v = product(m, rows, w), result(m, c, v), half(1);
+            if (order == 4) half(1), v = product(m, rows, w), half(0), result(m, c, v);
+            if (order == 5) half(1), v = product(m, rows, w), result(m, c, v), half(0);
+            for (int i = 0; i < GATHER; ++i) EXPECT(m[i] == want[i]);
+          }
+          // Nothing is copied for operands that lie apart.
+          if (std::abs(x - keep) >= L && std::abs(x - c) >= L && std::abs(keep - c) >= L && std::abs(keep - w) >= L) {
+            EXPECT(!plan.rows_aside && !plan.keep_first);
+          }
+        }
+      }
+    }
+  }
+  // No input buffer to fill: only a result over the rows takes them aside.
+  EXPECT(!plan_alone(Span{base, L}, Span{nullptr, 0}, Span{base + 4, L}, Span{base + 8, L}).keep_first);
+  EXPECT(!plan_alone(Span{base, L}, Span{nullptr, 0}, Span{base + 4, L}, Span{base + 8, L}).rows_aside);
+  EXPECT(plan_alone(Span{base, L}, Span{nullptr, 0}, Span{base + 4, L}, Span{base + 3, L}).rows_aside);
+}
+
 int main(int argc, char **argv) {
   if (argc < 2) {
     std::fprintf(stderr, "usage: %s <scratch directory>\n", argv[0]);
@@ -371,6 +439,7 @@ int main(int argc, char **argv) {
   test_allreduce_selection();
   test_broadcast_plan();
   test_ep_config_limits();
+  test_fused_alone_plan();
   test_file_bootstrap_between_threads(argv[1]);
   if (g_failures) {
     std::fprintf(stderr, "%d check(s) failed\n", g_failures);

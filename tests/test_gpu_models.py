@@ -103,6 +103,7 @@ def test_tp_mlp_alone_reads_the_rows_where_they_are(shm, m):
     """A team of one: rows in ordinary memory, strided rows and results that share memory with an operand give what the
     input buffer gives, and the rows are the input buffer's content afterwards."""
     from rocshmem_b200.models import tp_mlp
+    from rocshmem_b200.ops import gemm
     d = 512
     mlp = tp_mlp.TensorParallelMLP(d, d, m, seed=4)
     x = (torch.randn(m, d, generator=torch.Generator().manual_seed(m)) * 0.5).to(torch.bfloat16).cuda()
@@ -120,6 +121,25 @@ def test_tp_mlp_alone_reads_the_rows_where_they_are(shm, m):
     mlp.tp.ag_gemm(mlp.w_gate_up, out=mlp.input_buffer(), swiglu=True)
     assert torch.equal(mlp.input_buffer(), h)
     assert torch.equal(mlp.tp.gemm_rs(h, mlp.w_down, out=h), want)
+    # The rows given, and the result over the input buffer, or rows and input buffer sharing some of their memory: the
+    # rows become the buffer's content first, then the result is written.
+    hidden = mlp.tp.ag_gemm(mlp.w_gate_up, swiglu=True, x=x)
+    for rep in range(3):
+        mlp.tp.ag_gemm(mlp.w_gate_up, out=mlp.input_buffer(), swiglu=True, x=x)
+        assert torch.equal(mlp.input_buffer(), hidden)
+    both = shm.zeros((m + 8, d), torch.bfloat16)
+    tp = gemm.TensorParallelLinear(m)
+    own = tp._ag_buffers(d)[0]
+    tp._ag_buffers(d)[0] = both[:m]
+    for first in (0, 8):
+        both[8:].copy_(x)
+        got = tp.ag_gemm(mlp.w_gate_up, out=both[first:first + m], swiglu=True, x=both[8:])
+        assert torch.equal(got, hidden)
+        assert first == 0 or torch.equal(both[:8], x[:8])
+    clean(shm)
+    tp._ag_buffers(d)[0] = own
+    tp.destroy()
+    shm.free(both)
     # A call on another stream than the current one.
     side = torch.cuda.Stream()
     torch.cuda.synchronize()
