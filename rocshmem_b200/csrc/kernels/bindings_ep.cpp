@@ -65,9 +65,11 @@ void bind_ep(py::module_ &m) {
       .def_readonly("epoch", &EpHandle::epoch)
       .def("dispatch", [](EpHandle &h, uintptr_t x, uintptr_t topk_idx, uintptr_t topk_w, int num_tokens,
                           uintptr_t stream, uintptr_t zero_y) {
-        h.epoch += 1;
+        // A call that is refused launches nothing, so it does not count: the kernels' grid barriers and parities follow
+        // the epoch.
         check(ep_dispatch(reinterpret_cast<rocshmem_team_t>(h.team), h.cfg, h.buf, P<void>(x), P<int>(topk_idx),
-                          P<float>(topk_w), num_tokens, h.epoch, P<void>(stream), P<void>(zero_y)), "ep_dispatch");
+                          P<float>(topk_w), num_tokens, h.epoch + 1, P<void>(stream), P<void>(zero_y)), "ep_dispatch");
+        h.epoch += 1;
       }, py::arg("x"), py::arg("topk_idx"), py::arg("topk_w"), py::arg("num_tokens"), py::arg("stream"),
            py::arg("zero_y") = 0)
       .def("combine", [](EpHandle &h, uintptr_t y, uintptr_t out, uintptr_t topk_idx, uintptr_t topk_w,

@@ -200,6 +200,8 @@ class EpDispatcher:
         for t in (x, topk_idx, topk_weights):
             if not t.is_contiguous():
                 raise ValueError("dispatch: tensors must be contiguous")
+        if zero_result and not (self.low_latency and self.n_ranks == 1):
+            raise ValueError("dispatch: zero_result needs low-latency mode and a team of one")
         with trace_range("rocshmem_b200.ep_dispatch"):
             self._h.dispatch(x.data_ptr(), topk_idx.data_ptr(), topk_weights.data_ptr(), T, _stream(stream),
                              self.result_buffer().data_ptr() if zero_result else 0)

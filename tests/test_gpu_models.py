@@ -216,3 +216,21 @@ def test_moe_feed_forward_low_latency_alone(shm, quantize, T):
         assert gemm.gemm_error_count() == before
         assert (out - want).abs().max().item() <= 5e-2 * want.abs().max().item() + 0.05
     layer.destroy()
+
+
+@pytest.mark.parametrize("dynamic", [False, True])
+def test_refused_zero_result_leaves_the_dispatcher_usable(shm, dynamic):
+    """zero_result belongs to low-latency mode: elsewhere it is refused, and the calls after it work."""
+    from rocshmem_b200.ops import moe
+    T, E, K, H = 40, 8, 2, 512
+    x = torch.randn(T, H, generator=torch.Generator().manual_seed(1)).to(torch.bfloat16).cuda()
+    idx, w = (t.cuda() for t in moe.make_routing(T, E, K, 3))
+    d = moe.EpDispatcher(E, K, H, T, quantize=False, dynamic=dynamic)
+    for rep in range(3):
+        with pytest.raises(ValueError):
+            d.dispatch(x, idx, w, zero_result=True)
+        r = d.dispatch(x, idx, w)
+        clean(shm)
+        assert r.num_rows() == T and torch.equal(r.recv_x[:T], x)
+        assert torch.equal(r.rows_per_expert()[:E].long(), torch.bincount(idx.flatten().long(), minlength=E))
+    d.destroy()

@@ -286,3 +286,24 @@ def test_unknown_comparison_is_refused_at_once(shm4):
         with pytest.raises(ValueError, match="comparison"):
             call()
     assert time.time() - t0 < 2          # not after a time-out
+
+
+def test_refused_dispatch_leaves_the_dispatcher_as_it_was(shm4):
+    """The kernels' grid barriers and parities follow the number of launches: a call that is refused is not one."""
+    from rocshmem_b200 import _native
+    from rocshmem_b200.ops import moe
+    C = _native.load()
+    team = shm4.team_world()
+    h = C.EpHandle(team.handle, 16, 2, 512, 8, 1, 0, 4, 0, 0, 0, {})
+    for tokens, zero_y in ((9, 0), (8, 4096)):        # more tokens than the buffers hold; zero_y outside low-latency mode
+        with pytest.raises(RuntimeError):
+            h.dispatch(0, 0, 0, tokens, 0, zero_y)
+        assert h.epoch == 0
+    # and in Python, before anything is allocated for the call
+    for low_latency, ranks in ((False, 1), (True, 4), (False, 4)):
+        d = object.__new__(moe.EpDispatcher)
+        d.max_tokens, d.hidden, d.top_k, d.low_latency, d.n_ranks, d._h, d._y = 8, 512, 2, low_latency, ranks, h, None
+        with pytest.raises(ValueError, match="zero_result"):
+            d.dispatch(torch.zeros(8, 512, dtype=torch.bfloat16), torch.zeros(8, 2, dtype=torch.int32), torch.zeros(8, 2),
+                       stream=0, zero_result=True)
+        assert h.epoch == 0 and d._y is None
