@@ -19,6 +19,27 @@ def _stream(stream) -> int:
     return stream.cuda_stream if hasattr(stream, "cuda_stream") else int(stream)
 
 
+def _copy_on(stream, dst: torch.Tensor, src: torch.Tensor) -> None:
+    """``dst.copy_(src)`` in the order of ``stream``: after what has been queued there (earlier calls that still read
+    ``dst``) and after the work of the current stream, which made ``src``."""
+    cur = torch.cuda.current_stream(dst.device)
+    handle = _stream(stream)
+    if handle == cur.cuda_stream:
+        dst.copy_(src)
+        return
+    default = torch.cuda.default_stream(dst.device)
+    own = default if handle in (default.cuda_stream, 1) else torch.cuda.ExternalStream(handle, device=dst.device)
+    with torch.cuda.stream(cur):
+        capturing = torch.cuda.is_current_stream_capturing()
+    with torch.cuda.stream(own):
+        # Between a stream that is being captured and one that is not there is no order to express.
+        if torch.cuda.is_current_stream_capturing() == capturing:
+            own.wait_stream(cur)
+        dst.copy_(src)
+    if src.is_cuda:
+        src.record_stream(own)
+
+
 def _check(t: torch.Tensor, name: str) -> None:
     if t.dtype != torch.bfloat16 or not t.is_contiguous() or not t.is_cuda:
         raise ValueError(f"{name} must be a contiguous bf16 CUDA tensor")
@@ -213,14 +234,15 @@ class TensorParallelLinear:
         keep = 0
         if x is not None:
             # With a team of one the kernel reads the rows where they are and copies them beside its arithmetic. Rows
-            # that the kernel cannot read as they are, or that the call's stream does not own, are copied first.
+            # that the kernel cannot read as they are, or that the call's stream does not own, are copied first, on the
+            # call's stream.
             if (self.n_ranks == 1 and x.dtype == torch.bfloat16 and x.shape == rows.shape and x.device == rows.device
                     and x.is_contiguous() and x.data_ptr() % 16 == 0 and not x.requires_grad
                     and _stream(stream) == torch.cuda.current_stream().cuda_stream):
                 if x.data_ptr() != rows.data_ptr():
                     rows, keep = x, rows.data_ptr()
             else:
-                rows.copy_(x)
+                _copy_on(stream, rows, x)
         buf[3] += 1
         if out is None:
             out = torch.empty((self.n_ranks * self.m_shard, N // 2 if swiglu else N), dtype=torch.bfloat16,

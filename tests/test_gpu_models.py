@@ -140,11 +140,29 @@ def test_tp_mlp_alone_reads_the_rows_where_they_are(shm, m):
     tp._ag_buffers(d)[0] = own
     tp.destroy()
     shm.free(both)
-    # A call on another stream than the current one.
+    # A call on another stream than the current one: in place where that stream is made current, else copied on it.
     side = torch.cuda.Stream()
     torch.cuda.synchronize()
     with torch.cuda.stream(side):
         out = mlp(x)
+    torch.cuda.synchronize()
+    assert torch.equal(out, want)
+    # The call's stream is busy with a call that still has to read the input buffer, and the rows are late.
+    other = (x.float() * 0.5).to(torch.bfloat16)
+    mlp.input_buffer().copy_(other)
+    want_other = mlp().clone()
+    late, first, out = (torch.empty_like(x) for _ in range(3))
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(20_000_000)          # about 10 ms
+    mlp(out=first, stream=side)                # the buffer holds `other`
+    torch.cuda._sleep(60_000_000)
+    late.copy_(x)
+    mlp(late, out=out, stream=side)
+    assert not side.query()
+    torch.cuda.synchronize()
+    assert torch.equal(first, want_other)
+    assert torch.equal(mlp.input_buffer(), x)
     clean(shm)
     assert torch.equal(out, want)
     mlp.destroy()
