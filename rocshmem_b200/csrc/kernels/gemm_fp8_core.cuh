@@ -26,6 +26,7 @@
 #include <cuda_fp8.h>
 
 #include "gemm_core.cuh"
+#include "gemm_select.hpp"
 #include "sm100_ptx.cuh"
 
 namespace rocshmem {
@@ -221,7 +222,7 @@ __device__ __forceinline__ void run(const CUtensorMap *map_a, const CUtensorMap 
       const float4 *sa4 = reinterpret_cast<const float4 *>((A_GATHER ? gather->scales : a_scale) + a_scale_row * k_blocks);
       // B's scales are the same for the whole warp, and one line holds 32 of them: they are read K block by K block, one
       // ahead (four ahead like A's, they cost the registers that made the SwiGLU kernels spill).
-      const float *sb = b_scale + static_cast<size_t>(t.b_row[SWIGLU ? 0 : half] / 128) * k_blocks;
+      const float *sb = b_scale + static_cast<size_t>(t.b_row[SWIGLU ? 0 : b_scale_box(half, t.cols)] / 128) * k_blocks;
       const float *su = b_scale + static_cast<size_t>(t.b_row[1] / 128) * k_blocks;
       // LATE_A: the A scales of a tile may still be on their way from another GPU until the producer has
       // seen the tile's rows arrive; the first finished K block proves it has. Read past L1 (__ldcg).

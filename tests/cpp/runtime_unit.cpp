@@ -22,6 +22,7 @@
 #include "../kernels/coll_select.hpp"
 #include "../kernels/ep_kernels.hpp"
 #include "../kernels/fused_select.hpp"
+#include "../kernels/gemm_select.hpp"
 
 using namespace rocshmem;
 
@@ -357,6 +358,27 @@ static void test_ep_config_limits() {
   EXPECT(ep_ll_combine_blocks(c) == ROCSHMEM_LIB_MAX_BLOCKS);
 }
 
+// Block-scaled GEMM: the rows of B's scale array that the two halves of a tile read exist, in every group and for every
+// width that is accepted (a multiple of 128), and are the half's own where it has columns.
+static void test_b_scale_rows() {
+  using namespace rocshmem::kernels;
+  for (int groups = 1; groups <= 3; ++groups) {
+    for (int n = 128; n <= 2048; n += 128) {
+      for (int g = 0; g < groups; ++g) {
+        for (int first = 0; first < n; first += 256) {
+          const int b_row[2] = {g * n + first, g * n + first + 128};
+          const int cols = n - first < 256 ? n - first : 256;
+          for (int half = 0; half < 2; ++half) {
+            const int row = b_row[b_scale_box(half, cols)] / 128;
+            EXPECT(row < groups * n / 128);
+            if (half * 128 < cols) EXPECT(row == (g * n + first) / 128 + half);
+          }
+        }
+      }
+    }
+  }
+}
+
 // all-gather -> GEMM on a team of one: what the plan does gives the buffers that the documented order gives (the rows become
 // the input buffer's content, then the result is written), wherever the operands lie. The "GEMM" of this model reads the
 // weight and the rows it is given when the kernel runs, and writes two result bytes; inside the kernel the reads, the copy
@@ -440,6 +462,7 @@ int main(int argc, char **argv) {
   test_broadcast_plan();
   test_ep_config_limits();
   test_fused_alone_plan();
+  test_b_scale_rows();
   test_file_bootstrap_between_threads(argv[1]);
   if (g_failures) {
     std::fprintf(stderr, "%d check(s) failed\n", g_failures);

@@ -377,3 +377,19 @@ def test_gemm_fp8_few_tiles(m, n, k):
     size = (a_deq.double().abs() @ b_deq.double().abs().t())       # what the rounding of the sums scales with
     assert ((out.double() - want).abs() <= 2 ** -8 * want.abs() + 2 ** -17 * size).all()
     assert torch.equal(gemm.gemm_fp8_blockscaled(a_q, a_s, b_q, b_s), out)
+
+
+@pytest.mark.parametrize("m,n", [(300, 128 * 149), (9000, 384)])
+def test_gemm_fp8_last_tile_of_half_width(m, n):
+    """A width that is an odd multiple of 128, with too many tiles for the split kernel: the last column tile has no
+    second half, and its scales are not read."""
+    from rocshmem_b200.ops import gemm
+    k = 512
+    a_q, a_s, b_q, b_s, a_deq, b_deq = _fp8_inputs(m, n, k, seed=n)
+    before = gemm.gemm_error_count()
+    out = gemm.gemm_fp8_blockscaled(a_q, a_s, b_q, b_s)
+    torch.cuda.synchronize()
+    assert gemm.gemm_error_count() == before
+    want = a_deq.double() @ b_deq.double().t()
+    size = a_deq.double().abs() @ b_deq.double().abs().t()         # what the rounding of the sums scales with
+    assert ((out.double() - want).abs() <= 2 ** -8 * want.abs() + 2 ** -17 * size).all()
