@@ -708,13 +708,13 @@ int ag_gemm_fp8(rocshmem_team_t team, const void *x_q, const float *x_s, void *g
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int sms = device_sm_count();
-  auto launch = [&](auto kernel) -> int {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, gemm8::SMEM_BYTES);
-    if (e != cudaSuccess) return static_cast<int>(e);
+  auto launch = [&](auto kernel, int rc) -> int {
+    if (rc != 0) return rc;
     return launch_pes(kernel, sms, gemm8::THREADS, gemm8::SMEM_BYTES, s, !alone, map_a, map_b, a);
   };
-  if (c_q != nullptr) return launch(ag_gemm_fp8_kernel<true, true>);
-  return swiglu ? launch(ag_gemm_fp8_kernel<true>) : launch(ag_gemm_fp8_kernel<false>);
+  if (c_q != nullptr) return launch(ag_gemm_fp8_kernel<true, true>, gemm8::prepare<ag_gemm_fp8_kernel<true, true>>());
+  return swiglu ? launch(ag_gemm_fp8_kernel<true>, gemm8::prepare<ag_gemm_fp8_kernel<true>>())
+                : launch(ag_gemm_fp8_kernel<false>, gemm8::prepare<ag_gemm_fp8_kernel<false>>());
 }
 
 int gemm_rs_fp8(rocshmem_team_t team, const void *a_q, const float *a_scale, const void *b_q, const float *b_scale,
@@ -738,8 +738,7 @@ int gemm_rs_fp8(rocshmem_team_t team, const void *a_q, const float *a_scale, con
                                overlaps(out, out_bytes, b_scale, size_t(n / 128) * (k / 128) * sizeof(float)));
   RsArgs a{team, static_cast<__nv_bfloat16 *>(staging), static_cast<__nv_bfloat16 *>(aside ? staging : out), m_shard, n,
            k, alone ? nullptr : grid_counter, epoch};
-  cudaError_t e = cudaFuncSetAttribute(gemm_rs_fp8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, gemm8::SMEM_BYTES);
-  if (e != cudaSuccess) return static_cast<int>(e);
+  if (int rc = gemm8::prepare<gemm_rs_fp8_kernel>()) return rc;
   if (int rc = launch_pes(gemm_rs_fp8_kernel, device_sm_count(), gemm8::THREADS, gemm8::SMEM_BYTES,
                           static_cast<cudaStream_t>(stream), !alone, map_a, map_b, a_scale, b_scale, a)) {
     return rc;

@@ -192,12 +192,6 @@ grouped_gemm_fp8_scatter_kernel(const __grid_constant__ CUtensorMap map_a, const
   gemm8::run<false, false, true, false>(&map_a, &map_b, a_scale, b_scale, k / gemm8::KB, sched, epi, smem_raw, sh);
 }
 
-template <typename K>
-int prepare8(K kernel) {
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, gemm8::SMEM_BYTES);
-  return e == cudaSuccess ? 0 : static_cast<int>(e);
-}
-
 }  // namespace
 
 int fp8_error_count() {
@@ -220,7 +214,7 @@ int gemm_fp8_blockscaled(const void *a_q, const float *a_scale, const void *b_q,
   if (!encode_tmap_2d(&map_a, a_q, m, k, 1, gemm8::BM) || !encode_tmap_2d(&map_b, b_q, n, k, 1, gemm8::BN / 2)) return -1;
   const int tiles = ((m + gemm8::BM - 1) / gemm8::BM) * ((n + gemm8::BN - 1) / gemm8::BN);
   const int grid = std::min(tiles, device_sm_count());
-  if (int rc = prepare8(gemm_fp8_kernel)) return rc;
+  if (int rc = gemm8::prepare<gemm_fp8_kernel>()) return rc;
   gemm_fp8_kernel<<<grid, gemm8::THREADS, gemm8::SMEM_BYTES, static_cast<cudaStream_t>(stream)>>>(
       map_a, map_b, a_scale, b_scale, static_cast<__nv_bfloat16 *>(c), m, n, k);
   return cudaGetLastError();
@@ -240,13 +234,14 @@ int grouped_gemm_fp8_blockscaled(const void *a_q, const float *a_scale, const vo
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int grid = device_sm_count();
-  auto launch = [&](auto kernel) -> int {
-    if (int rc = prepare8(kernel)) return rc;
+  auto launch = [&](auto kernel, int rc) -> int {
+    if (rc != 0) return rc;
     kernel<<<grid, gemm8::THREADS, gemm8::SMEM_BYTES, s>>>(map_a, map_b, a_scale, b_scale,
                                                            static_cast<__nv_bfloat16 *>(c), offsets, groups, n, k);
     return cudaGetLastError();
   };
-  return swiglu ? launch(grouped_gemm_fp8_kernel<true>) : launch(grouped_gemm_fp8_kernel<false>);
+  return swiglu ? launch(grouped_gemm_fp8_kernel<true>, gemm8::prepare<grouped_gemm_fp8_kernel<true>>())
+                : launch(grouped_gemm_fp8_kernel<false>, gemm8::prepare<grouped_gemm_fp8_kernel<false>>());
 }
 
 int grouped_gemm_fp8_swiglu_quant(const void *a_q, const float *a_scale, const int *row_index, const void *b_q,
@@ -264,11 +259,11 @@ int grouped_gemm_fp8_swiglu_quant(const void *a_q, const float *a_scale, const i
   gemm::GatherSrc src{row_index, static_cast<const unsigned char *>(a_q), static_cast<size_t>(k), a_scale, k / 128};
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (row_index != nullptr) {
-    if (int rc = prepare8(grouped_gemm_fp8_swiglu_quant_kernel<true>)) return rc;
+    if (int rc = gemm8::prepare<grouped_gemm_fp8_swiglu_quant_kernel<true>>()) return rc;
     grouped_gemm_fp8_swiglu_quant_kernel<true><<<device_sm_count(), gemm8::THREADS, gemm8::SMEM_BYTES, s>>>(
         map_a, map_b, a_scale, b_scale, static_cast<unsigned char *>(out_q), out_s, offsets, groups, n, k, src);
   } else {
-    if (int rc = prepare8(grouped_gemm_fp8_swiglu_quant_kernel<false>)) return rc;
+    if (int rc = gemm8::prepare<grouped_gemm_fp8_swiglu_quant_kernel<false>>()) return rc;
     grouped_gemm_fp8_swiglu_quant_kernel<false><<<device_sm_count(), gemm8::THREADS, gemm8::SMEM_BYTES, s>>>(
         map_a, map_b, a_scale, b_scale, static_cast<unsigned char *>(out_q), out_s, offsets, groups, n, k, src);
   }
@@ -287,7 +282,7 @@ int grouped_gemm_fp8_scatter_add(const void *a_q, const float *a_scale, const vo
       !encode_tmap_2d(&map_b, b_q, static_cast<uint64_t>(groups) * n, k, 1, gemm8::BN / 2)) {
     return -1;
   }
-  if (int rc = prepare8(grouped_gemm_fp8_scatter_kernel)) return rc;
+  if (int rc = gemm8::prepare<grouped_gemm_fp8_scatter_kernel>()) return rc;
   grouped_gemm_fp8_scatter_kernel<<<device_sm_count(), gemm8::THREADS, gemm8::SMEM_BYTES,
                                     static_cast<cudaStream_t>(stream)>>>(
       map_a, map_b, a_scale, b_scale, static_cast<__nv_bfloat16 *>(y), offsets, row_index, weights, groups, n, k);

@@ -25,6 +25,8 @@
 #include <cuda_bf16.h>
 #include <cuda_fp8.h>
 
+#include <atomic>
+
 #include "gemm_core.cuh"
 #include "gemm_select.hpp"
 #include "sm100_ptx.cuh"
@@ -49,7 +51,10 @@ constexpr int GATHER_WARPS = 2;                         // warps 2 and 3
 constexpr int THREADS = (FIRST_ACC_WARP + ACC_WARPS) * 32;
 // Registers per thread: what 384 threads are launched with, and what the two parts of the block hold while they work.
 constexpr int REGS_LAUNCH = 168, REGS_FEED = 72, REGS_ACC = 216;
-static_assert(4 * REGS_FEED + ACC_WARPS * REGS_ACC <= (4 + ACC_WARPS) * REGS_LAUNCH, "setmaxnreg.inc would wait for ever");
+constexpr bool registers_fit(int compiled) {
+  return hand_over_fits(compiled, REGS_LAUNCH, FIRST_ACC_WARP, REGS_FEED, ACC_WARPS, REGS_ACC);
+}
+static_assert(registers_fit(REGS_LAUNCH), "setmaxnreg.inc would wait for ever");
 constexpr int TMEM_COLS = 512;
 constexpr unsigned long long WAIT_BUDGET_NS = gemm::WAIT_BUDGET_NS;
 
@@ -76,7 +81,8 @@ struct Shared {
 // A_GATHER: the A rows (and their scales) are picked by index: tile row r reads row gather->row_index[t.a_row + r]
 // of gather->base / gather->scales. Warps 2 and 3 copy the rows into the stage with the 128-byte swizzle (cp.async)
 // instead of a TMA load.
-// The kernel is compiled for and launched with THREADS threads (__launch_bounds__(THREADS, 1): REGS_LAUNCH registers).
+// The kernel is compiled for and launched with THREADS threads (__launch_bounds__(THREADS, 1): REGS_LAUNCH registers),
+// after prepare<Kernel>().
 template <bool SWIGLU, bool LATE_A = false, bool EPI_ADD = false, bool QUANT_OUT = false, bool A_GATHER = false,
           class Scheduler, class Epilogue>
 __device__ __forceinline__ void run(const CUtensorMap *map_a, const CUtensorMap *map_b, const float *a_scale,
@@ -393,6 +399,23 @@ __device__ __forceinline__ void run(const CUtensorMap *map_a, const CUtensorMap 
     sm100::tmem_dealloc(tmem_base, TMEM_COLS);
   }
   if (threadIdx.x == 0 && sh.abort_flag) atomicAdd(&gemm::g_gemm_errors, 1u);
+}
+
+// Before every launch of a kernel of this core. One that was compiled to another number of registers (a register cap,
+// another compiler) is refused here, because its setmaxnreg would wait without a limit; that is asked once.
+template <auto Kernel>
+inline int prepare() {
+  static std::atomic<int> fits{-1};   // -1: not asked yet. Every thread would find the same.
+  int ok = fits.load(std::memory_order_relaxed);
+  if (ok < 0) {
+    cudaFuncAttributes attr;
+    const cudaError_t e = cudaFuncGetAttributes(&attr, Kernel);
+    if (e != cudaSuccess) return static_cast<int>(e);
+    ok = registers_fit(attr.numRegs) ? 1 : 0;
+    fits.store(ok, std::memory_order_relaxed);
+  }
+  if (ok == 0) return static_cast<int>(cudaErrorInvalidKernelImage);
+  return static_cast<int>(cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
 }
 
 }  // namespace gemm8

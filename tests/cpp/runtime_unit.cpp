@@ -379,6 +379,18 @@ static void test_b_scale_rows() {
   }
 }
 
+// Registers handed over inside a block: only a kernel that was compiled to the number the shares were laid out for is
+// launched, and only if the shares fit it.
+static void test_register_hand_over() {
+  using namespace rocshmem::kernels;
+  EXPECT(hand_over_fits(168, 168, 4, 72, 8, 216));
+  for (int compiled = 24; compiled <= 255; ++compiled) {
+    if (compiled != 168) EXPECT(!hand_over_fits(compiled, 168, 4, 72, 8, 216));
+  }
+  EXPECT(!hand_over_fits(168, 168, 4, 80, 8, 216));
+  EXPECT(!hand_over_fits(160, 160, 4, 72, 8, 216));
+}
+
 // all-gather -> GEMM on a team of one: what the plan does gives the buffers that the documented order gives (the rows become
 // the input buffer's content, then the result is written), wherever the operands lie. The "GEMM" of this model reads the
 // weight and the rows it is given when the kernel runs, and writes two result bytes; inside the kernel the reads, the copy
@@ -463,6 +475,7 @@ int main(int argc, char **argv) {
   test_ep_config_limits();
   test_fused_alone_plan();
   test_b_scale_rows();
+  test_register_hand_over();
   test_file_bootstrap_between_threads(argv[1]);
   if (g_failures) {
     std::fprintf(stderr, "%d check(s) failed\n", g_failures);
