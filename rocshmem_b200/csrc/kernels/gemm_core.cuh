@@ -22,6 +22,7 @@
 
 #include <type_traits>
 
+#include "silu.cuh"
 #include "sm100_ptx.cuh"
 
 namespace rocshmem {
@@ -126,18 +127,6 @@ struct Shared {
   uint32_t tmem_base;
   volatile int abort_flag;
 };
-
-// x / (1 + exp(-x)) without the branches of the IEEE division: the approximate reciprocal, and one Newton correction of
-// the quotient (the remainder x - d q is exact up to one rounding), which leaves at most the last bit. Where the correction
-// would meet inf * 0 (d past the reciprocal's range, x infinite) the uncorrected quotient is the answer: -0, inf or NaN.
-// With the IEEE form the block-scaled gate/up GEMM (16 experts, 7168 -> 2 x 2048) took 518 us for 1024 rows an expert and 117
-// for 64, with this one 505 and 107; the bf16 one for 64 rows 186 and 171.
-__device__ __forceinline__ float silu(float x) {
-  const float d = 1.0f + __expf(-x);
-  const float r = __fdividef(1.0f, d), q = x * r;
-  const float better = fmaf(fmaf(-d, q, x), r, q);
-  return d < 8e37f && x < 3e38f ? better : q;
-}
 
 // Scheduler: struct with  __device__ bool get(int iter, Tile &t)  (false: no more tiles for this CTA),
 //                         __device__ bool ready(const Tile &t)    (producer-side hook, bounded; false aborts)

@@ -13,12 +13,21 @@
 #include <cuda_runtime.h>
 
 #include "kernels/launch.cuh"
+#include "kernels/silu.cuh"
 #include "rocshmem/rocshmem.h"
 
 namespace py = pybind11;
 using namespace rocshmem;
 
 namespace {
+
+// The SwiGLU epilogues' activation, and the same with CUDA's division.
+__global__ void silu_kernel(const float *x, float *got, float *want, int n) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    got[i] = kernels::gemm::silu(x[i]);
+    want[i] = x[i] / (1.0f + __expf(-x[i]));
+  }
+}
 
 enum RmaOp { RMA_PUT = 0, RMA_PUT_NBI, RMA_GET, RMA_GET_NBI, RMA_P, RMA_G };
 enum ScopeSel { SC_THREAD = 0, SC_WARP, SC_BLOCK };
@@ -706,6 +715,11 @@ PYBIND11_MODULE(_testk, m) {
   m.def("barrier_stress", [](uintptr_t slots, int rounds, uintptr_t errors, int threads, uintptr_t stream) {
     ok(kernels::launch_pes(barrier_kernel, 1, threads, 0, S(stream), false, P<long long>(slots), rounds,
                            P<int>(errors)), "barrier_kernel");
+  });
+  m.def("silu", [](uintptr_t x, uintptr_t got, uintptr_t want, int n, uintptr_t stream) {
+    silu_kernel<<<256, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+        reinterpret_cast<const float *>(x), reinterpret_cast<float *>(got), reinterpret_cast<float *>(want), n);
+    if (cudaGetLastError() != cudaSuccess) throw std::runtime_error("silu");
   });
   m.def("shmem_ptr", [](uintptr_t buf, int offset, uintptr_t stream) {
     ok(kernels::launch_pes(ptr_kernel, 1, 32, 0, S(stream), false, P<char>(buf), offset), "ptr_kernel");

@@ -393,3 +393,27 @@ def test_gemm_fp8_last_tile_of_half_width(m, n):
     want = a_deq.double() @ b_deq.double().t()
     size = a_deq.double().abs() @ b_deq.double().abs().t()         # what the rounding of the sums scales with
     assert ((out.double() - want).abs() <= 2 ** -8 * want.abs() + 2 ** -17 * size).all()
+
+
+def test_silu_against_cuda_division():
+    """The epilogues' quotient against CUDA's correctly rounded division of the same operands: at most the last bit
+    apart, and the same zeros, infinities and NaNs, over all bf16 values, all magnitudes of fp32 and the range in which
+    1 + exp(-x) is more than 2^126."""
+    from rocshmem_b200 import _native
+    g = torch.Generator().manual_seed(5)
+    every_bf16 = (torch.arange(65536, dtype=torch.int64) << 16).to(torch.int32).view(torch.float32)
+    every_exponent = torch.randint(-2 ** 31, 2 ** 31, (1 << 20,), generator=g).to(torch.int32).view(torch.float32)
+    x = torch.cat([every_bf16, every_exponent, torch.linspace(-110, 110, 1 << 20),
+                   torch.linspace(-88.8, -87.2, 1 << 18), torch.tensor([float("inf"), -float("inf"), float("nan"), 0.0, -0.0])])
+    x = x.cuda()
+    got, want = torch.empty_like(x), torch.empty_like(x)
+    _native.load_test_kernels().silu(x.data_ptr(), got.data_ptr(), want.data_ptr(), x.numel(),
+                                     torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    assert torch.equal(got.isnan(), want.isnan())
+    number = ~want.isnan()
+    got, want = got[number].view(torch.int32).long(), want[number].view(torch.int32).long()
+    apart = (got - want).abs()
+    assert apart.max().item() <= 1
+    special = (want & 0x7FFFFFFF == 0) | (want & 0x7FFFFFFF == 0x7F800000)
+    assert apart[special].max().item() == 0
