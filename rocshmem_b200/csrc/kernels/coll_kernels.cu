@@ -434,14 +434,16 @@ fcollect_nvls_kernel(rocshmem_team_t team, char *dest_arg, const char *source_ar
 
 // ---- copies -----------------------------------------------------------------------------------------------
 
-// A block's part of a push, whole 16-byte vectors: `n` destinations in the order member(0), member(1), ...; those with
-// the same source are served from one read of it. Eight loads of 16 bytes a thread are in flight (a block of 512 threads
-// and 64 KiB a SM: with four, and a read of the source for every destination, four PEs on one GPU gathered 16 MiB each in
-// 110 us, 3 TB/s).
-template <bool ONE_SOURCE, class Source, class Dest>
+// A block's part of a push, whole 16-byte vectors, to `n` destinations in the order member(0), member(1), ... Eight loads
+// of 16 bytes a thread are in flight (a block of 512 threads and 64 KiB a SM).
+// INTERLEAVED: all destinations have the same source and are served batch by batch from one read of it. That is for PEs
+// that share one GPU and so its HBM: four of them gathered 16 MiB each in 110 us (3 TB/s) with four loads in flight and a
+// read for every destination, in 81 us so. Over NVLink, where the links bound a push and not the reads, it has not been
+// measured: there a block sends its whole share to one destination before the next, the members in rotated order.
+template <bool INTERLEAVED, class Source, class Dest>
 __device__ __forceinline__ void push_vectors(int n, size_t nvec, Source source, Dest dest) {
   constexpr int U = 8;
-  if (ONE_SOURCE) {
+  if (INTERLEAVED) {
     const int4 *from = source(0);
     for (size_t v = threadIdx.x; v < nvec; v += size_t(U) * blockDim.x) {
       int4 r[U];
@@ -462,6 +464,7 @@ __device__ __forceinline__ void push_vectors(int n, size_t nvec, Source source, 
     for (int d = 0; d < n; ++d) {
       const int4 *from = source(d);
       int4 *to = dest(d);
+      if (to == nullptr) continue;
       for (size_t v = threadIdx.x; v < nvec; v += size_t(U) * blockDim.x) {
         int4 r[U];
 #pragma unroll
@@ -512,8 +515,9 @@ push_kernel(rocshmem_team_t team, char *dest_arg, const char *source_arg, size_t
       return reinterpret_cast<int4 *>(remote_ptr(to, team_pe_to_world(t, j)));
     };
     if (vectors && hi > lo) {
-      if (mode == 2) push_vectors<false>(n, (hi - lo) / 16, vec_source, vec_dest);
-      else push_vectors<true>(n, (hi - lo) / 16, vec_source, vec_dest);
+      const bool one_gpu = gridDim.z > 1;   // several PEs in this process
+      if (mode != 2 && one_gpu) push_vectors<true>(n, (hi - lo) / 16, vec_source, vec_dest);
+      else push_vectors<false>(n, (hi - lo) / 16, vec_source, vec_dest);
     }
     detail::Group<detail::Scope::BLOCK> g;
     for (int d = 0; d < n && hi > lo && !vectors; ++d) {

@@ -1,12 +1,13 @@
 """The library's allreduce and push kernels by team size and payload: teams of up to four and of more members
-take different reduction loops, payloads that are whole 16-byte vectors another copy than others."""
+take different reduction loops, payloads that are whole 16-byte vectors another copy than others, and a process with one
+PE another order of the destinations than one with several."""
 import pytest
 import torch
 
 pytestmark = pytest.mark.gpu
 
 
-@pytest.fixture(scope="module", params=[2, 3, 4, 6, 8])
+@pytest.fixture(scope="module", params=[1, 2, 3, 4, 6, 8])
 def shm(request):
     import rocshmem_b200 as s
     if s.is_initialized():
