@@ -23,6 +23,7 @@
 #include <algorithm>
 #include <atomic>
 
+#include "fused_select.hpp"
 #include "gemm2_core.cuh"
 #include "gemm_core.cuh"
 #include "sm100_ptx.cuh"
@@ -300,7 +301,9 @@ inline int split_for(long long tiles, int k_slabs, int bn, int least) {
   return least <= 1 && tiles <= clusters_at_once<Kernel>(1, bn) ? 1 : 0;
 }
 
-// Runs the product if it has few enough tiles; returns -2 if not, else 0, a cudaError_t, or -1 when the driver cannot
+// Runs the product if it has few enough tiles and its result shares no memory with an operand (the persistent kernels
+// compute up to 128 x 256 or 256 x 256 results in one piece, which reads all of A and B before it writes; here a
+// neighbouring tile may still be reading); returns -2 if not, else 0, a cudaError_t, or -1 when the driver cannot
 // encode tensor maps. `least`: 1 for bf16; 2 for e4m3, where a tile of half the width costs the accumulate warps more
 // than half the time (1024 x 2048 x 4096 as 128 tiles of one CTA: 25 us, as 64 of the persistent kernel's 21). `Wide` and `Narrow` are run<FP8, 128> and run<FP8, 64> behind __launch_bounds__(threads(BN), 1);
 // narrow tiles are taken where they keep more CTAs busy (64 x 2048: 16 wide tiles x 4 CTAs, 32 narrow ones x 4).
@@ -308,11 +311,8 @@ inline int split_for(long long tiles, int k_slabs, int bn, int least) {
 template <auto Wide, auto Narrow, typename Encode>
 inline int try_launch(const void *a, const void *b, void *c, const float *a_scale,
                       const float *b_scale, int m, int n, int k_bytes, int least, Encode encode, cudaStream_t stream) {
-  cudaError_t e = cudaFuncSetAttribute(Wide, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT);
-  if (e == cudaSuccess) {
-    e = cudaFuncSetAttribute(Narrow, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT);
-  }
-  if (e != cudaSuccess) return static_cast<int>(e);
+  const Span result{c, size_t(m) * n * 2};
+  if (overlaps(result, Span{a, size_t(m) * k_bytes}) || overlaps(result, Span{b, size_t(n) * k_bytes})) return -2;
   Args args{static_cast<__nv_bfloat16 *>(c), a_scale, b_scale, m, n, (k_bytes + SLAB_BYTES - 1) / SLAB_BYTES, 0, 0,
             m < BM ? (m + 7) / 8 * 8 : BM, 0};
   const long long row_blocks = (m + BM - 1) / BM, wide_tiles = row_blocks * ((n + 127) / 128),

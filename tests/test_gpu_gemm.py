@@ -417,3 +417,23 @@ def test_silu_against_cuda_division():
     assert apart.max().item() <= 1
     special = (want & 0x7FFFFFFF == 0) | (want & 0x7FFFFFFF == 0x7F800000)
     assert apart[special].max().item() == 0
+
+
+@pytest.mark.parametrize("two_cta", [None, False])
+def test_gemm_bf16_result_over_an_operand(two_cta):
+    """A product of one tile of the persistent kernels may be written over an operand: it reads all before it writes."""
+    from rocshmem_b200.ops import gemm
+    g = torch.Generator(device="cuda").manual_seed(3)
+    n = 256
+    b = (torch.randn(n, n, generator=g, device="cuda") * n ** -0.5).to(torch.bfloat16)
+    for m in (1, 100, 128) + ((256,) if two_cta is None else ()):
+        a = torch.randn(m, n, generator=g, device="cuda").to(torch.bfloat16)
+        want = gemm.gemm_bf16(a, b)
+        for rep in range(3):
+            over = a.clone()
+            assert gemm.gemm_bf16(over, b, out=over, two_cta=two_cta) is over
+            assert torch.allclose(over.float(), want.float(), rtol=2 ** -7, atol=2 ** -23 * n)   # two roundings to bf16
+        if m == n:
+            over = b.clone()
+            gemm.gemm_bf16(a, over, out=over)
+            assert torch.allclose(over.float(), want.float(), rtol=2 ** -7, atol=2 ** -23 * n)
