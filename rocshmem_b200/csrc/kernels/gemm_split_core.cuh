@@ -264,13 +264,22 @@ __device__ __forceinline__ void run(const CUtensorMap *map_a, const CUtensorMap 
   if (threadIdx.x == 0 && sh.abort_flag) atomicAdd(&gemm::g_gemm_errors, 1u);
 }
 
+template <auto Kernel>
+inline cudaError_t allow_smem() {
+  return cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT);
+}
+
 // How many clusters of `split` CTAs the GPU runs at once (a cluster stays inside a GPC, so 15 of eight and 33 of four
-// on 148 SMs), asked once for each size. 0: not at all.
+// on 148 SMs), asked until it is answered, once for each size. 0: not at all.
 template <auto Kernel>
 inline int clusters_at_once(int split, int bn) {
-  static std::atomic<int> known[MAX_SPLIT + 1] = {};   // 0: not asked yet. Every thread would find the same.
-  int n = known[split].load(std::memory_order_relaxed);
+  static std::atomic<int> known[MAX_SPLIT + 1] = {};   // answer + 1; 0: none yet. Every thread would find the same.
+  const int n = known[split].load(std::memory_order_relaxed);
   if (n == 0) {
+    if (allow_smem<Kernel>() != cudaSuccess) {
+      cudaGetLastError();
+      return 0;
+    }
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = static_cast<unsigned>(split);
@@ -284,12 +293,12 @@ inline int clusters_at_once(int split, int bn) {
     int found = 0;
     if (cudaOccupancyMaxActiveClusters(&found, Kernel, &cfg) != cudaSuccess) {
       cudaGetLastError();
-      found = 0;
+      return 0;
     }
-    n = found > 0 ? found : -1;
-    known[split].store(n, std::memory_order_relaxed);
+    known[split].store(found + 1, std::memory_order_relaxed);
+    return found;
   }
-  return n > 0 ? n : 0;
+  return n - 1;
 }
 // CTAs that share each of `tiles` tiles: as many as run at once, each with at least four K slabs. 0: more tiles than the
 // GPU takes at once, or fewer CTAs a tile than `least`: the persistent kernels with their larger tiles are better.
@@ -344,6 +353,8 @@ inline int try_launch(const void *a, const void *b, void *c, const float *a_scal
   cfg.stream = stream;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
+  const cudaError_t e = take_narrow ? allow_smem<Narrow>() : allow_smem<Wide>();
+  if (e != cudaSuccess) return static_cast<int>(e);
   return static_cast<int>(cudaLaunchKernelEx(&cfg, take_narrow ? Narrow : Wide, map_a, map_b, args));
 }
 
