@@ -243,12 +243,13 @@ class TensorParallelLinear:
                     rows, keep = x, rows.data_ptr()
             else:
                 _copy_on(stream, rows, x)
-        buf[3] += 1
         if out is None:
             out = torch.empty((self.n_ranks * self.m_shard, N // 2 if swiglu else N), dtype=torch.bfloat16,
                               device=w.device)
+        # The counters of the exchange follow the number of launches: a call that is refused is not one.
         rt._C().ag_gemm_bf16(self.team.handle, rows.data_ptr(), gathered.data_ptr(), flags.data_ptr(), w.data_ptr(),
-                             out.data_ptr(), self.m_shard, N, K, buf[3], int(swiglu), _stream(stream), keep)
+                             out.data_ptr(), self.m_shard, N, K, buf[3] + 1, int(swiglu), _stream(stream), keep)
+        buf[3] += 1
         self.kernel_launches += 1
         return out
 
@@ -265,11 +266,11 @@ class TensorParallelLinear:
             self._rs[N] = [rt.zeros((self.n_ranks, self.m_shard, N), torch.bfloat16), rt.zeros(16, torch.int64), 0]
         entry = self._rs[N]
         staging, counter = entry[0], entry[1]
-        entry[2] += 1
         if out is None:
             out = torch.empty((self.m_shard, N), dtype=torch.bfloat16, device=a.device)
         rt._C().gemm_rs_bf16(self.team.handle, a.data_ptr(), w.data_ptr(), staging.data_ptr(), out.data_ptr(),
-                             self.m_shard, N, K, counter.data_ptr(), entry[2], _stream(stream))
+                             self.m_shard, N, K, counter.data_ptr(), entry[2] + 1, _stream(stream))
+        entry[2] += 1
         self.kernel_launches += 1
         return out
 
@@ -394,13 +395,13 @@ class TensorParallelLinearFp8:
         """All-gather of the quantised activations fused with ``gathered @ w.T`` (block-scaled e4m3), optionally with SwiGLU."""
         N, K = w_q.shape
         x_q, x_s, g_q, g_s, flags, _ = buf = self._ag_buffers(K)
-        buf[5] += 1
         if out is None:
             out = torch.empty((self.n_ranks * self.m_shard, N // 2 if swiglu else N), dtype=torch.bfloat16,
                               device=w_q.device)
         rt._C().ag_gemm_fp8(self.team.handle, x_q.data_ptr(), x_s.data_ptr(), g_q.data_ptr(), g_s.data_ptr(),
                             flags.data_ptr(), w_q.data_ptr(), w_s.data_ptr(), out.data_ptr(), self.m_shard, N, K,
-                            buf[5], int(swiglu), _stream(stream))
+                            buf[5] + 1, int(swiglu), _stream(stream))
+        buf[5] += 1
         self.kernel_launches += 1
         return out
 
@@ -413,10 +414,10 @@ class TensorParallelLinearFp8:
         if tuple(out_q.shape) != (self.n_ranks * self.m_shard, N // 2) or tuple(out_s.shape) != (out_q.shape[0], N // 256):
             raise ValueError("ag_gemm_quantized: out shapes")
         x_q, x_s, g_q, g_s, flags, _ = buf = self._ag_buffers(K)
-        buf[5] += 1
         rt._C().ag_gemm_fp8(self.team.handle, x_q.data_ptr(), x_s.data_ptr(), g_q.data_ptr(), g_s.data_ptr(),
-                            flags.data_ptr(), w_q.data_ptr(), w_s.data_ptr(), 0, self.m_shard, N, K, buf[5], 1,
+                            flags.data_ptr(), w_q.data_ptr(), w_s.data_ptr(), 0, self.m_shard, N, K, buf[5] + 1, 1,
                             _stream(stream), out_q.data_ptr(), out_s.data_ptr())
+        buf[5] += 1
         self.kernel_launches += 1
 
     def gemm_rs(self, a_q: torch.Tensor, a_s: torch.Tensor, w_q: torch.Tensor, w_s: torch.Tensor,
@@ -429,11 +430,11 @@ class TensorParallelLinearFp8:
             # staging slices of every rank's partial of my rows, and the grid counter's 128 bytes
             self._rs[N] = [rt.zeros((self.n_ranks, self.m_shard, N), torch.bfloat16), rt.zeros(16, torch.int64), 0]
         entry = self._rs[N]
-        entry[2] += 1
         if out is None:
             out = torch.empty((self.m_shard, N), dtype=torch.bfloat16, device=a_q.device)
         rt._C().gemm_rs_fp8(self.team.handle, a_q.data_ptr(), a_s.data_ptr(), w_q.data_ptr(), w_s.data_ptr(),
-                            entry[0].data_ptr(), out.data_ptr(), self.m_shard, N, K, entry[1].data_ptr(), entry[2],
+                            entry[0].data_ptr(), out.data_ptr(), self.m_shard, N, K, entry[1].data_ptr(), entry[2] + 1,
                             _stream(stream))
+        entry[2] += 1
         self.kernel_launches += 1
         return out

@@ -307,3 +307,35 @@ def test_refused_dispatch_leaves_the_dispatcher_as_it_was(shm4):
             d.dispatch(torch.zeros(8, 512, dtype=torch.bfloat16), torch.zeros(8, 2, dtype=torch.int32), torch.zeros(8, 2),
                        stream=0, zero_result=True)
         assert h.epoch == 0 and d._y is None
+
+
+def test_refused_tensor_parallel_calls_leave_the_counters(monkeypatch):
+    """The exchange's counters follow the number of launches, so a refused call of the fused GEMMs must not count: the
+    next one would wait for rows that nobody sends."""
+    from rocshmem_b200.ops import gemm
+
+    class Refuses:
+        def __getattr__(self, name):
+            def fn(*args):
+                raise RuntimeError(name)
+            return fn
+    monkeypatch.setattr(gemm.rt, "_C", lambda: Refuses())
+    t = lambda *shape: torch.zeros(*shape, dtype=torch.bfloat16)
+    monkeypatch.setattr(gemm, "_check", lambda *a: None)
+    monkeypatch.setattr(gemm, "_check8", lambda *a: None)
+
+    class Team:
+        handle = 0
+    for cls, ag, rs in ((gemm.TensorParallelLinear, [t(8, 8)] * 3 + [7], [t(1, 8, 8), t(16), 7]),
+                        (gemm.TensorParallelLinearFp8, [t(8, 8)] * 5 + [7], [t(1, 8, 8), t(16), 7])):
+        tp = object.__new__(cls)
+        tp.team, tp.n_ranks, tp.m_shard, tp._ag, tp._rs, tp.kernel_launches = Team(), 1, 8, {8: ag}, {8: rs}, 0
+        fp8 = cls is gemm.TensorParallelLinearFp8
+        calls = [lambda: tp.ag_gemm(*([t(8, 8)] * (2 if fp8 else 1)), stream=0),
+                 lambda: tp.gemm_rs(*([t(8, 8)] * (4 if fp8 else 2)), stream=0)]
+        if fp8:
+            calls.append(lambda: tp.ag_gemm_quantized(t(256, 8), t(8, 8), t(8, 128), t(8, 1), stream=0))
+        for call in calls:
+            with pytest.raises(RuntimeError):
+                call()
+            assert ag[-1] == 7 and rs[-1] == 7 and tp.kernel_launches == 0
