@@ -86,7 +86,9 @@ class EpDispatcher:
                  low_latency: bool = False):
         """``dynamic``: dispatch hands (token, destination) pairs to warps through per-destination counters and
         combine hands tokens out through a counter (levels the tail when fixed shares carry unequal numbers of
-        bytes; dispatch pays a second grid barrier for it). ``None`` takes ``ROCSHMEM_EP_DYNAMIC`` (default on).
+        bytes; dispatch pays a second grid barrier for it). ``None`` takes ``ROCSHMEM_EP_DYNAMIC`` (default on). On a
+        team of one, where all shares are equal, and in low-latency mode there is nothing to hand out: the attribute
+        ``dynamic`` is then False.
 
         ``expert_layout``: the dispatch kernel also groups the received (row, k) pairs by local expert
         (:meth:`expert_pairs`), which a grouped GEMM consumes directly.
@@ -121,7 +123,7 @@ class EpDispatcher:
             self.blocks *= 2
         if dynamic is None:
             dynamic = os.environ.get("ROCSHMEM_EP_DYNAMIC", "1") not in ("", "0")
-        self.dynamic = bool(dynamic) and not self.low_latency
+        self.dynamic = bool(dynamic) and not self.low_latency and P > 1
         self.with_expert_layout = bool(expert_layout)
         rows = P * max_tokens
         z = rt.zeros

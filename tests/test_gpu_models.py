@@ -244,6 +244,7 @@ def test_refused_zero_result_leaves_the_dispatcher_usable(shm, dynamic):
     x = torch.randn(T, H, generator=torch.Generator().manual_seed(1)).to(torch.bfloat16).cuda()
     idx, w = (t.cuda() for t in moe.make_routing(T, E, K, 3))
     d = moe.EpDispatcher(E, K, H, T, quantize=False, dynamic=dynamic)
+    assert not d.dynamic and not hasattr(d, "stage_meta")      # nothing to hand out on a team of one
     for rep in range(3):
         with pytest.raises(ValueError):
             d.dispatch(x, idx, w, zero_result=True)
