@@ -94,7 +94,7 @@ def bench_tp_mlp(args, world, rank, res):
         torch.cuda.synchronize()
         err8 = (out8.float() - ref.float()).abs().max().item()
         t8 = timed(lambda: mlp8(x), args.iters)
-        t8_ag = timed(lambda: mlp8.tp.ag_gemm(mlp8.w1_q, mlp8.w1_s, out=mlp8.h, swiglu=True), args.iters)
+        t8_ag = timed(lambda: mlp8.tp.ag_gemm_quantized(mlp8.w1_q, mlp8.w1_s, mlp8.h_q, mlp8.h_s), args.iters)
         t8_rs = timed(lambda: mlp8.tp.gemm_rs(mlp8.h_q, mlp8.h_s, mlp8.w2_q, mlp8.w2_s), args.iters)
         res["tp_mlp_fp8"] = {"fused_us": t8, "ag_gemm_us": t8_ag, "gemm_rs_us": t8_rs, "speedup_vs_nccl_cublas_bf16": t_base / t8,
                              "tflops_per_gpu": flops / t8 / 1e6, "max_abs_diff_vs_bf16_baseline": err8,

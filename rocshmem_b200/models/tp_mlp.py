@@ -86,7 +86,6 @@ class TensorParallelMLPFp8:
         self.w1_q, self.w1_s = gemm.quantize_weight_128x128(w1)
         self.w2_q, self.w2_s = gemm.quantize_weight_128x128(w2)
         M = P * m_shard
-        self.h = torch.empty((M, self.ff_local), dtype=torch.bfloat16, device=dev)
         self.h_q = torch.empty((M, self.ff_local), dtype=torch.uint8, device=dev)
         self.h_s = torch.empty((M, self.ff_local // 128), dtype=torch.float32, device=dev)
 
@@ -110,7 +109,8 @@ class TensorParallelMLPFp8:
 
 
 def reference_forward_fp8(x_full: torch.Tensor, n_ranks: int, d_model: int, d_ff: int, seed: int = 0) -> torch.Tensor:
-    """fp32 evaluation of :class:`TensorParallelMLPFp8` with the same quantisation points."""
+    """fp32 evaluation of :class:`TensorParallelMLPFp8` with the same quantisation points: the input shard, the hidden
+    activation (from its fp32 values) and the weights; each rank's partial product is rounded to bf16."""
     from ..ops import moe
     q, s = moe.ref_quantize_1x128(x_full.cpu())
     x = moe.ref_dequantize_1x128(q, s).float()
@@ -121,8 +121,7 @@ def reference_forward_fp8(x_full: torch.Tensor, n_ranks: int, d_model: int, d_ff
         w1d = gemm.dequantize_weight_128x128(*gemm.quantize_weight_128x128(w1))
         w2d = gemm.dequantize_weight_128x128(*gemm.quantize_weight_128x128(w2))
         hc = x @ w1d.t()
-        h = (torch.nn.functional.silu(hc[:, :ff]) * hc[:, ff:]).to(torch.bfloat16)
-        hq, hs = moe.ref_quantize_1x128(h)
+        hq, hs = moe.ref_quantize_1x128(torch.nn.functional.silu(hc[:, :ff]) * hc[:, ff:])
         out += (moe.ref_dequantize_1x128(hq, hs).float() @ w2d.t()).to(torch.bfloat16).float()
     return out
 
