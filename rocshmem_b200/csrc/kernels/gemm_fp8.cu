@@ -205,7 +205,8 @@ int gemm_fp8_blockscaled(const void *a_q, const float *a_scale, const void *b_q,
   // K blocks are consumed four at a time; B scale blocks cover 128 rows of B.
   if (m <= 0 || n <= 0 || k <= 0 || (k % 512) != 0 || (n % 128) != 0) return cudaErrorInvalidValue;
   CUtensorMap map_a, map_b;
-  // As many 128 x 128 tiles as SMs at most: clusters that share a tile's K.
+  // Few tiles: clusters of at least two CTAs that share a tile's K, so about half as many 128 x 128 tiles as SMs at most,
+  // and a K of 1024 or more.
   const int rc = gemms::try_launch<gemm_fp8_split_kernel<128>, gemm_fp8_split_kernel<64>>(
       a_q, b_q, c, a_scale, b_scale, m, n, k, 2,
       [k](CUtensorMap *map, const void *base, int rows, int box) { return encode_tmap_2d(map, base, rows, k, 1, box); },

@@ -270,9 +270,9 @@ int gemm_bf16_pair(const void *a, const void *b, void *c, int m, int n, int k, v
 
 int gemm_bf16_one_cta(const void *a, const void *b, void *c, int m, int n, int k, void *stream);
 
-// As many 128 x 128 tiles as SMs at most: clusters that share a tile's K (gemm_split_core.cuh). More tiles, and more
-// than one 128-row block: two CTAs per 256 x 256 tile (about 10 % faster, see gemm2_core.cuh), unless
-// ROCSHMEM_GEMM_TWO_CTA=0 asks for the one-CTA kernel.
+// As many 128 x 128 tiles as SMs at most: clusters that share a tile's K (gemm_split_core.cuh), whatever
+// ROCSHMEM_GEMM_TWO_CTA says. More tiles, and more than one 128-row block: two CTAs per 256 x 256 tile (about 10 %
+// faster, see gemm2_core.cuh), unless ROCSHMEM_GEMM_TWO_CTA=0 asks for the one-CTA kernel.
 int gemm_bf16(const void *a, const void *b, void *c, int m, int n, int k, void *stream) {
   static const bool two_cta = [] {
     const char *e = std::getenv("ROCSHMEM_GEMM_TWO_CTA");

@@ -314,7 +314,8 @@ inline int split_for(long long tiles, int k_slabs, int bn, int least) {
 // compute up to 128 x 256 or 256 x 256 results in one piece, which reads all of A and B before it writes; here a
 // neighbouring tile may still be reading); returns -2 if not, else 0, a cudaError_t, or -1 when the driver cannot
 // encode tensor maps. `least`: 1 for bf16; 2 for e4m3, where a tile of half the width costs the accumulate warps more
-// than half the time (1024 x 2048 x 4096 as 128 tiles of one CTA: 25 us, as 64 of the persistent kernel's 21). `Wide` and `Narrow` are run<FP8, 128> and run<FP8, 64> behind __launch_bounds__(threads(BN), 1);
+// than half the time (1024 x 2048 x 4096 as 128 tiles of one CTA: 25 us, as 64 of the persistent kernel's 21). `Wide` and
+// `Narrow` are run<FP8, 128> and run<FP8, 64> behind __launch_bounds__(threads(BN), 1);
 // narrow tiles are taken where they keep more CTAs busy (64 x 2048: 16 wide tiles x 4 CTAs, 32 narrow ones x 4).
 // `encode(map, base, rows, box_rows)` makes the K-slab map of an operand.
 template <auto Wide, auto Narrow, typename Encode>
@@ -333,7 +334,7 @@ inline int try_launch(const void *a, const void *b, void *c, const float *a_scal
   const int bn = take_narrow ? 64 : 128;
   args.tiles_n = (n + bn - 1) / bn;
   args.split = take_narrow ? ns : ws;
-  // The ring takes what shared memory is left: a decode step is bound by the bytes in flight (32 x 7168 x 8192 bf16: ten
+  // The ring takes what shared memory is left: a decode step is bound by the bytes in flight (32 x 7168 x 8192 bf16: eleven
   // stages of 20 KiB). Behind it lies what an MMA reads past a short last stage (128 rows of A), in front the alignment.
   const int stage_bytes = (args.a_box_rows + bn) * SLAB_BYTES;
   const int overrun = std::max(0, BM * SLAB_BYTES - stage_bytes);

@@ -50,8 +50,9 @@ def _check(t: torch.Tensor, name: str) -> None:
 def gemm_bf16(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None, stream=None,
               two_cta: Optional[bool] = None) -> torch.Tensor:
     """``a [M, K] @ b [N, K].T -> [M, N]`` (bf16 in, fp32 accumulate in TMEM, bf16 out). By default the
-    library picks the kernel (a pair of CTAs per 256 x 256 tile, ``tcgen05`` ``cta_group::2``, when M > 128);
-    ``two_cta`` forces one or the other."""
+    library picks the kernel: clusters that share a tile's K for products with few tiles, else a pair of CTAs per 256 x
+    256 tile (``tcgen05`` ``cta_group::2``) when M > 128, else one CTA per 128 x 256 tile. ``two_cta`` forces one or the
+    other of the last two."""
     _check(a, "a")
     _check(b, "b")
     M, K = a.shape
