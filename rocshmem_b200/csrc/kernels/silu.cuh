@@ -6,18 +6,17 @@ namespace kernels {
 namespace gemm {
 
 // x / (1 + exp(-x)) without the branches of the IEEE division: the approximate reciprocal, and one Newton correction of
-// the quotient (the remainder x - d q is exact up to one rounding), which leaves at most the last bit. Past 2^126 the
-// approximate reciprocal of d is 0, so a quarter of both operands is divided there. Where the quotient is exact, or the
-// remainder is no number (d or x infinite), the quotient stands as it is: a zero with its sign, inf or NaN.
+// the quotient (the remainder x - d q is exact up to one rounding), which leaves at most the last bit. The reciprocal is
+// taken of a quarter of d = 1 + exp(-x), because that of a number past 2^126 would be flushed to 0. Where the quotient is
+// exact, or the remainder is no number (d or x infinite), the quotient stands as it is: a zero with its sign, inf or NaN.
 // With the IEEE form the block-scaled gate/up GEMM (16 experts, 7168 -> 2 x 2048) took 518 us for 1024 rows an expert and 117
 // for 64, with this one 505 and 107; the bf16 one for 64 rows 186 and 171.
 __device__ __forceinline__ float silu(float x) {
-  float d = 1.0f + __expf(-x);
-  const float s = d > 8e37f ? 0.25f : 1.0f;
-  d *= s;
-  x *= s;
-  const float r = __fdividef(1.0f, d), q = x * r;
-  const float rest = fmaf(-d, q, x);
+  const float e = __expf(-x), d = 1.0f + e;
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(fmaf(0.25f, e, 0.25f)));
+  r *= 0.25f;
+  const float q = x * r, rest = fmaf(-d, q, x);
   return fabsf(rest) > 0.f ? fmaf(rest, r, q) : q;
 }
 
