@@ -167,8 +167,8 @@ struct AgScheduler {
       t.c_col = j0;
     } else {
       t.b_row[0] = nt * gemm::BN;
-      t.b_row[1] = nt * gemm::BN + gemm::BN / 2;
       t.cols = min(gemm::BN, n - nt * gemm::BN);
+      t.b_row[1] = second_box(t.b_row[0], t.cols);
       t.c_col = nt * gemm::BN;
     }
     t.c_row = t.a_row;
@@ -333,8 +333,8 @@ struct RsScheduler {
     t.a_row = owner * m_shard + mt * gemm::BM;
     t.rows = gemm::BM;
     t.b_row[0] = nt * gemm::BN;
-    t.b_row[1] = nt * gemm::BN + gemm::BN / 2;
     t.cols = min(gemm::BN, n - nt * gemm::BN);
+    t.b_row[1] = second_box(t.b_row[0], t.cols);
     t.c_row = mt * gemm::BM;   // row inside the owner's shard
     t.c_col = nt * gemm::BN;
     t.tag = owner;

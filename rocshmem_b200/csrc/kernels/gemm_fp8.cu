@@ -25,9 +25,9 @@ struct PlainScheduler8 {
     gemm::raster(id, tiles / tiles_n, tiles_n, gemm::RASTER_GROUP, mt, nt);
     t.a_row = mt * gemm8::BM;
     t.b_row[0] = nt * gemm8::BN;
-    t.b_row[1] = nt * gemm8::BN + gemm8::BN / 2;
     t.rows = min(gemm8::BM, m - t.a_row);
     t.cols = min(gemm8::BN, n - nt * gemm8::BN);
+    t.b_row[1] = second_box(t.b_row[0], t.cols);
     t.c_row = t.a_row;
     t.c_col = nt * gemm8::BN;
     return true;
@@ -93,8 +93,8 @@ struct GroupedScheduler8 {
           t.c_col = j0;
         } else {
           t.b_row[0] = g * n + nt * gemm8::BN;
-          t.b_row[1] = t.b_row[0] + gemm8::BN / 2;
           t.cols = min(gemm8::BN, n - nt * gemm8::BN);
+          t.b_row[1] = second_box(t.b_row[0], t.cols);
           t.c_col = nt * gemm8::BN;
         }
         return true;

@@ -229,7 +229,7 @@ __device__ __forceinline__ void run(const CUtensorMap *map_a, const CUtensorMap 
       // B's scales are the same for the whole warp, and one line holds 32 of them: they are read K block by K block, one
       // ahead. Four ahead, like A's, they cost registers: the quantising SwiGLU kernels then spilled 68 (stores) / 76 (loads)
       // and, with gathered rows, 104 / 124 bytes; so they spill 20 / 36 and 56 / 92.
-      const float *sb = b_scale + static_cast<size_t>(t.b_row[SWIGLU ? 0 : b_scale_box(half, t.cols)] / 128) * k_blocks;
+      const float *sb = b_scale + static_cast<size_t>(t.b_row[SWIGLU ? 0 : half] / 128) * k_blocks;
       const float *su = b_scale + static_cast<size_t>(t.b_row[1] / 128) * k_blocks;
       // LATE_A: the A scales of a tile may still be on their way from another GPU until the producer has
       // seen the tile's rows arrive; the first finished K block proves it has. Read past L1 (__ldcg).

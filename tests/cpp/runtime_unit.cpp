@@ -366,10 +366,10 @@ static void test_b_scale_rows() {
     for (int n = 128; n <= 2048; n += 128) {
       for (int g = 0; g < groups; ++g) {
         for (int first = 0; first < n; first += 256) {
-          const int b_row[2] = {g * n + first, g * n + first + 128};
           const int cols = n - first < 256 ? n - first : 256;
+          const int b_row[2] = {g * n + first, second_box(g * n + first, cols)};
           for (int half = 0; half < 2; ++half) {
-            const int row = b_row[b_scale_box(half, cols)] / 128;
+            const int row = b_row[half] / 128;
             EXPECT(row < groups * n / 128);
             if (half * 128 < cols) EXPECT(row == (g * n + first) / 128 + half);
           }
