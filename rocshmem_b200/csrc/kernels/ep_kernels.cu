@@ -681,6 +681,7 @@ __global__ void __launch_bounds__(kEpThreads, 1) ep_dispatch_kernel(DispatchArgs
 
 constexpr unsigned kLlThreads = 128;
 
+template <bool ALONE>
 __global__ void __launch_bounds__(kLlThreads) ep_ll_dispatch_kernel(DispatchArgs a) {
   __shared__ int s_e[EP_MAX_TOPK];
   __shared__ int s_rank[EP_MAX_TOPK];
@@ -754,7 +755,7 @@ __global__ void __launch_bounds__(kLlThreads) ep_ll_dispatch_kernel(DispatchArgs
       sent_slot[size_t(tok) * P + tid] = slot;
     }
     __syncthreads();
-    if (a.zero_y != nullptr && s_slot[0] >= 0) {
+    if (ALONE && a.zero_y != nullptr && s_slot[0] >= 0) {
       int4 *y = reinterpret_cast<int4 *>(static_cast<__nv_bfloat16 *>(rebase(a.zero_y)) + size_t(s_slot[0]) * H);
       for (unsigned v = tid; v < unsigned(H / 8); v += nthr) y[v] = make_int4(0, 0, 0, 0);
     }
@@ -811,12 +812,11 @@ __global__ void __launch_bounds__(kLlThreads) ep_ll_dispatch_kernel(DispatchArgs
   __syncthreads();
   // A rank on its own hands its rows to nobody but itself: fences of this GPU's scope do, and no signal has to be released.
   // (With the pair lists below: 128 tokens of 7168 in 11.5 us instead of 18.9, a call in a loop 15.1 instead of 22.6.)
-  const bool alone = P == 1;
   if (tid == 0) {
-    alone ? __threadfence() : __threadfence_system();  // this block's rows, before the count
+    ALONE ? __threadfence() : __threadfence_system();  // this block's rows, before the count
     const unsigned long long prev = atomicAdd(work + EP_WORK_LL_DONE, 1ull);
     s_last = (prev == gridDim.x - 1) ? 1 : 0;
-    if (s_last) alone ? __threadfence() : __threadfence_system();
+    if (s_last) ALONE ? __threadfence() : __threadfence_system();
   }
   __syncthreads();
   if (!s_last) return;
@@ -831,20 +831,20 @@ __global__ void __launch_bounds__(kLlThreads) ep_ll_dispatch_kernel(DispatchArgs
   __syncthreads();
   if (tid < unsigned(P)) {
     const unsigned long long c = __ldcg(work + EP_WORK_LL_ROWS + tid);
-    if (alone) {
+    if (ALONE) {
       detail::st_relaxed_sys(cnt_in, pack(epoch, static_cast<unsigned>(c)));
     } else {
-    // Release: the rows of all blocks (ordered before this store through the done counter and the fences around
-    // it) and the expert counts above are visible to whoever acquires the word.
-    detail::st_release_sys(remote_ptr(cnt_in + me * P + tid, team_pe_to_world(t, tid)),
-                           pack(epoch, static_cast<unsigned>(c)));
+      // Release: the rows of all blocks (ordered before this store through the done counter and the fences around
+      // it) and the expert counts above are visible to whoever acquires the word.
+      detail::st_release_sys(remote_ptr(cnt_in + me * P + tid, team_pe_to_world(t, tid)),
+                             pack(epoch, static_cast<unsigned>(c)));
     }
     work[EP_WORK_LL_ROWS + tid] = 0;
   }
   if (tid == 0) work[EP_WORK_LL_DONE] = 0;
   // Receive side: the signal of source s says how many rows it sent and that they have landed.
   bool ok = true;
-  if (alone) {
+  if (ALONE) {
     __threadfence();      // the other blocks' rows, counted above
   } else if (tid < unsigned(P)) {
     wait_packed(cnt_in + tid * P + me, epoch, tid, &ok);
@@ -1123,10 +1123,9 @@ int ep_dispatch(rocshmem_team_t team, const EpConfig &cfg, const EpBuffers &buf,
     if (buf.work_counter == nullptr) return cudaErrorInvalidValue;
     // A block per token; with several PEs per process the launch is cooperative and must fit the GPU at once.
     unsigned blocks = static_cast<unsigned>(std::max(1, std::min(num_tokens, 4096)));
-    if (rt.n_local() > 1) {
-      blocks = std::min(blocks, coresident_blocks_per_pe(ep_ll_dispatch_kernel, kLlThreads, 0, rt.n_local()));
-    }
-    return launch_pes(ep_ll_dispatch_kernel, blocks, kLlThreads, 0, static_cast<cudaStream_t>(stream), false, a);
+    auto kernel = ht->world.size == 1 ? ep_ll_dispatch_kernel<true> : ep_ll_dispatch_kernel<false>;
+    if (rt.n_local() > 1) blocks = std::min(blocks, coresident_blocks_per_pe(kernel, kLlThreads, 0, rt.n_local()));
+    return launch_pes(kernel, blocks, kLlThreads, 0, static_cast<cudaStream_t>(stream), false, a);
   }
   const int tpb = (cfg.max_tokens + cfg.blocks - 1) / cfg.blocks;
   const size_t smem = size_t(tpb) * ((ht->world.size + cfg.top_k) * sizeof(int) + sizeof(unsigned long long));
