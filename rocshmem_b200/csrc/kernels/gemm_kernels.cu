@@ -270,8 +270,8 @@ int gemm_bf16_pair(const void *a, const void *b, void *c, int m, int n, int k, v
 
 int gemm_bf16_one_cta(const void *a, const void *b, void *c, int m, int n, int k, void *stream);
 
-// As many 128 x 128 tiles as SMs at most: clusters that share a tile's K (gemm_split_core.cuh), whatever
-// ROCSHMEM_GEMM_TWO_CTA says. More tiles, and more than one 128-row block: two CTAs per 256 x 256 tile (about 10 %
+// Few tiles (half as many 128 x 128 ones as SMs at most, with one block of rows as many): clusters that share a tile's K
+// (gemm_split_core.cuh), whatever ROCSHMEM_GEMM_TWO_CTA says. More tiles, and more than one 128-row block: two CTAs per 256 x 256 tile (about 10 %
 // faster, see gemm2_core.cuh), unless ROCSHMEM_GEMM_TWO_CTA=0 asks for the one-CTA kernel.
 int gemm_bf16(const void *a, const void *b, void *c, int m, int n, int k, void *stream) {
   static const bool two_cta = [] {
@@ -280,7 +280,7 @@ int gemm_bf16(const void *a, const void *b, void *c, int m, int n, int k, void *
   }();
   if (m > 0 && n > 0 && k > 0 && k % 8 == 0) {
     const int rc = gemms::try_launch<gemm_bf16_split_kernel<128>, gemm_bf16_split_kernel<64>>(
-        a, b, c, nullptr, nullptr, m, n, k * 2, 1,
+        a, b, c, nullptr, nullptr, m, n, k * 2, split_least_bf16(m, k),
         [k](CUtensorMap *map, const void *base, int rows, int box) { return encode_tmap_2d(map, base, rows, k, 2, box); },
         static_cast<cudaStream_t>(stream));
     if (rc != -2) return rc;

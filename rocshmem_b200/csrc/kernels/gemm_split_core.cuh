@@ -26,6 +26,7 @@
 #include "fused_select.hpp"
 #include "gemm2_core.cuh"
 #include "gemm_core.cuh"
+#include "gemm_select.hpp"
 #include "sm100_ptx.cuh"
 
 namespace rocshmem {
@@ -313,9 +314,10 @@ inline int split_for(long long tiles, int k_slabs, int bn, int least) {
 // Runs the product if it has few enough tiles and its result shares no memory with an operand (the persistent kernels
 // compute up to 128 x 256 or 256 x 256 results in one piece, which reads all of A and B before it writes; here a
 // neighbouring tile may still be reading); returns -2 if not, else 0, a cudaError_t, or -1 when the driver cannot
-// encode tensor maps. `least`: 1 for bf16; 2 for e4m3, where a tile of half the width costs the accumulate warps more
-// than half the time (1024 x 2048 x 4096 as 128 tiles of one CTA: 25 us, as 64 of the persistent kernel's 21). `Wide` and
-// `Narrow` are run<FP8, 128> and run<FP8, 64> behind __launch_bounds__(threads(BN), 1);
+// encode tensor maps. `least`: see split_least_bf16; 2 for e4m3, where a tile of half the width costs the accumulate warps
+// more than half the time (96 to 144 tiles of one CTA against the persistent kernel's half as many, 256 to 2048 rows:
+// 5 - 19 % slower in all 36 shapes with a K of 512 to 4096, e.g. 512 x 4096 x 4096 24.7 us against 20.6, and within 3 %
+// at 7168). `Wide` and `Narrow` are run<FP8, 128> and run<FP8, 64> behind __launch_bounds__(threads(BN), 1);
 // narrow tiles are taken where they keep more CTAs busy (64 x 2048: 16 wide tiles x 4 CTAs, 32 narrow ones x 4).
 // `encode(map, base, rows, box_rows)` makes the K-slab map of an operand.
 template <auto Wide, auto Narrow, typename Encode>

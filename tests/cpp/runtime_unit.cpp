@@ -379,6 +379,14 @@ static void test_b_scale_rows() {
   }
 }
 
+// bf16 products with few tiles: one CTA a tile only for one block of rows and a K that is worth it.
+static void test_split_rule() {
+  using namespace rocshmem::kernels;
+  EXPECT(split_least_bf16(1, 1024) == 1 && split_least_bf16(128, 8192) == 1);
+  EXPECT(split_least_bf16(1, 1016) == 2 && split_least_bf16(128, 512) == 2);
+  EXPECT(split_least_bf16(129, 8192) == 2 && split_least_bf16(4096, 1024) == 2);
+}
+
 // Registers handed over inside a block: only a kernel that was compiled to the number the shares were laid out for is
 // launched, and only if the shares fit it.
 static void test_register_hand_over() {
@@ -475,6 +483,7 @@ int main(int argc, char **argv) {
   test_ep_config_limits();
   test_fused_alone_plan();
   test_b_scale_rows();
+  test_split_rule();
   test_register_hand_over();
   test_file_bootstrap_between_threads(argv[1]);
   if (g_failures) {
