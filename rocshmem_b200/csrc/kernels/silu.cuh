@@ -10,7 +10,8 @@ namespace gemm {
 // taken of a quarter of d = 1 + exp(-x), because that of a number past 2^126 would be flushed to 0. Where the quotient is
 // exact, or the remainder is no number (d or x infinite), the quotient stands as it is: a zero with its sign, inf or NaN.
 // With the IEEE form the block-scaled gate/up GEMM (16 experts, 7168 -> 2 x 2048) took 518 us for 1024 rows an expert and 117
-// for 64, with this one 505 and 107; the bf16 one for 64 rows 186 and 171.
+// for 64, with the reciprocal of d itself 505 and 107; the bf16 one for 64 rows 186 and 171. The quarter costs nothing that
+// the layers show (bf16 MoE layer, 1111 tokens: 222.0 us both ways).
 __device__ __forceinline__ float silu(float x) {
   const float e = __expf(-x), d = 1.0f + e;
   float r;
