@@ -36,7 +36,7 @@ def _copy_on(stream, dst: torch.Tensor, src: torch.Tensor) -> None:
         if torch.cuda.is_current_stream_capturing() == capturing:
             own.wait_stream(cur)
         dst.copy_(src)
-    if src.is_cuda:
+    if src.device == dst.device:   # from elsewhere torch orders and keeps the source itself
         src.record_stream(own)
 
 
